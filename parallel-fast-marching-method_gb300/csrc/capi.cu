@@ -498,11 +498,14 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         const int sgrid = stream_grid(fresh);
         if (nseg <= 0) nseg = stream_segments(ctx, nitems, nbx, nbz, sgrid, kStreamShapes[sidx].sx + kStreamShapes[sidx].sz - 2);
         nseg = std::min(nseg, g.nnr);
+        // (no empty segment: 130 layers in 16 segments of 9 fill only 15; an
+        // item above the grid would read parameters outside their arrays)
+        const int seg_len = (g.nnr + nseg - 1) / nseg;
+        nseg = (g.nnr + seg_len - 1) / seg_len;
         const fm3dt_ctx::Planes *PP = nullptr;
         int rc = ensure_block_planes(ctx, ctx->sweep_shape, nseg, &PP);
         if (rc) return rc;
         const auto &P = *PP;
-        const int seg_len = (g.nnr + nseg - 1) / nseg;
         // (items of one layer or column would miss a 2-deep neighbour)
         const bool track = !fresh && act_cur && seg_len >= 2 && kStreamShapes[sidx].sx >= 2;
         // One launch for the whole pass (FM_SWEEP_FLOW): items start as their
