@@ -1379,10 +1379,12 @@ int fm3dt_set_velocity(fm3dt_ctx *ctx, const double *velv)
     for (size_t q = 0; q < nvel; ++q)
         if (!(velv[q] > 0.0) || !std::isfinite(velv[q]))
             return fail(ctx, FM3DT_EINVAL, "velocity values must be positive and finite");
+    double *d_sums = nullptr;
+    DeviceScratch sc(ctx);
+    CK(sc.alloc(&d_sums, gridder_scratch(g)));
     CK(cudaMemcpyAsync(ctx->d_velv, velv, nvel * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    launch_gridder(g, ctx->d_velv, ctx->d_veln, ctx->stream);
-    launch_slowness(g, ctx->d_veln, ctx->d_s, ctx->prec, ctx->stream);
-    ctx->launches += 2;
+    launch_gridder(g, ctx->d_velv, ctx->d_veln, ctx->d_s, ctx->prec, d_sums, ctx->stream);
+    ctx->launches += 4;
     CKL();
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->have_velocity = 1;
@@ -1515,8 +1517,10 @@ int fm3dt_solve_point(fm3dt_ctx *ctx, int nev, const double *src, int refine, in
             CK(cudaMemcpyAsync(fc->d_velv, ctx->d_velv,
                                (size_t)(g.nvr + 2) * (g.nvx + 2) * (g.nvz + 2) * sizeof(double),
                                cudaMemcpyDeviceToDevice, fc->stream));
-            launch_gridder(fg, fc->d_velv, fc->d_veln, fc->stream);
-            launch_slowness(fg, fc->d_veln, fc->d_s, fc->prec, fc->stream);
+            DeviceScratch sc(fc);
+            double *d_sums = nullptr;
+            CK(sc.alloc(&d_sums, gridder_scratch(fg)));
+            launch_gridder(fg, fc->d_velv, fc->d_veln, fc->d_s, fc->prec, d_sums, fc->stream);
             fc->have_velocity = 1;
             // straight-ray start within two fine cells of the source
             int fb[6];
@@ -1532,11 +1536,10 @@ int fm3dt_solve_point(fm3dt_ctx *ctx, int nev, const double *src, int refine, in
             CK(cudaMemcpyAsync(fc->d_box, fb, sizeof fb, cudaMemcpyHostToDevice, fc->stream));
             CK(cudaMemcpyAsync(fc->d_box_init, fb, sizeof fb, cudaMemcpyHostToDevice, fc->stream));
             PointSource *d_src = nullptr;
-            DeviceScratch sc(fc);
             CK(sc.alloc(&d_src, 1));
             CK(cudaMemcpyAsync(d_src, &ps[e], sizeof(PointSource), cudaMemcpyHostToDevice, fc->stream));
             launch_point_analytic(fg, fc->prec, fc->d_veln, 1, d_src, fc->d_box, fc->d_T, fc->stream);
-            fc->launches += 4;
+            fc->launches += 6;
             fm3dt_status fst{};
             rc = solve_common(fc, 1, &fst, kPoint);
             ctx->launches += fc->launches;

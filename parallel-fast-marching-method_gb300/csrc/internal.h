@@ -182,8 +182,11 @@ inline int sweep_blocks_per_sm(int shape, int prec)
 }
 
 // model.cu
-void launch_gridder(const Geom &g, const double *velv, double *veln, cudaStream_t st);
-void launch_slowness(const Geom &g, const double *veln, void *s, int prec, cudaStream_t st);
+// padded velocity and interior slowness from the velocity nodes (four
+// launches); scratch: gridder_scratch(g) doubles
+size_t gridder_scratch(const Geom &g);
+void launch_gridder(const Geom &g, const double *velv, double *veln, void *s, int prec, double *scratch,
+                    cudaStream_t st);
 
 // boundary.cu
 struct PlaneWaveGeom { double rb, thc, phc, rbs; };
