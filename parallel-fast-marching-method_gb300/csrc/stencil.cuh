@@ -360,4 +360,322 @@ FM_HD R fm_update_upstream(R s, R tD, R tD2, R tX, R tX2, R tZ, R tZ2, bool inD,
     return tmin + best;
 }
 
+// ---------------------------------------------------------------------------
+// Double precision, screened in single precision
+// ---------------------------------------------------------------------------
+//
+// This GPU's double-precision pipe retires two lanes per SM and cycle, a
+// sixty-fourth of the single-precision rate, and bounds every double-precision
+// kernel: fm_update's eight octants take ~550 such operations a node (sixteen
+// quadratics, each with a square root and a division of ~8 operations).  The
+// node takes the least octant, so the octants are first solved in single
+// precision, and only those that can be the least -- one or two, mostly -- are
+// solved in double: the operations of the general update in its order, so
+// the same bits, ~60 double-precision operations a node.  Rounds of a two-event
+// 192x224x224 solve: 544 -> 161 ms, extra sweeps 146 -> 69 ms; the upstream-only
+// update of a 64^3 main sweep (latency of one warp's chain) 3.4 -> 1.9 ms.
+//
+// An octant's screened value stands when every decision on the way to it is
+// clear: each key differs from the solution it is compared with by more than
+// kScreen of it, no discriminant is below 1/32 of its positive part, and no
+// two keys so near that the sort could go the other way lead to different
+// terms.  Terms are formed relative to tmin, discriminants as
+//     a s^2 - sum_{i<j} w_i w_j (e_i - e_j)^2
+// (the same b^2 - a c without its cancellation), so a value that stands is
+// within ~1e-5 of the double-precision one (sqrt and division are within a few
+// ulp, and a discriminant's relative error is at most ~32 times its terms');
+// kScreen is twenty times that.  With m the least value that stands, an octant
+// is solved in double unless it stands above m (1 + 2 kScreen), or starts
+// there: its solution lies above its earliest key, every e being at least its
+// key and the root above their weighted mean.  An octant whose three terms
+// clearly all enter skips the pair's root too (it only decides that).
+constexpr float kScreen = 1.0f / 4096.0f;
+
+FM_HD unsigned long long fm_ubits(double v)
+{
+#ifdef __CUDA_ARCH__
+    return (unsigned long long)__double_as_longlong(v);
+#else
+    unsigned long long b;
+    __builtin_memcpy(&b, &v, sizeof b);
+    return b;
+#endif
+}
+// a < b of times (zero or above, +inf when unset; a NaN of either sign, as
+// copied from outside the grid, is above all), on the integer pipe
+FM_HD bool fm_less(double a, double b) { return fm_ubits(a) < fm_ubits(b); }
+
+// A time difference (zero or above, or +inf) rounded down to single
+// precision, on the integer pipe.
+FM_HD float fm_narrow(double v)
+{
+    const unsigned long long b = fm_ubits(v);
+    int h = (int)(b >> 32) - (896 << 20);            // exponent bias 1023 -> 127
+    unsigned lo = (unsigned)b >> 29;
+    if (h < 0) { h = 0; lo = 0; }
+    if (h >= (255 << 20)) { h = 255 << 20; lo = 0; }
+    const unsigned f = ((unsigned)h << 3) | lo;
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(f);
+#else
+    float r;
+    __builtin_memcpy(&r, &f, sizeof r);
+    return r;
+#endif
+}
+
+// One term of an octant: key, e, spacing and weight, in single precision.
+struct ScreenTerm {
+    float k, e, g, w;
+};
+
+// An octant's (or subset's) screened value: x; whether it stands; whether all
+// three terms enter; its earliest key.
+struct Screened {
+    float x, k0;
+    bool stands, three;
+};
+
+FM_HD void fm_screen_swap(ScreenTerm &a, ScreenTerm &b)
+{
+    const bool p = b.k < a.k;
+    const ScreenTerm t = a;
+    a.k = p ? b.k : a.k; a.e = p ? b.e : a.e; a.g = p ? b.g : a.g; a.w = p ? b.w : a.w;
+    b.k = p ? t.k : b.k; b.e = p ? t.e : b.e; b.g = p ? t.g : b.g; b.w = p ? t.w : b.w;
+}
+
+// a, b, c sorted by key
+FM_HD Screened fm_screen(float s, float s2, const ScreenTerm &a, const ScreenTerm &b, const ScreenTerm &c)
+{
+    Screened r;
+    r.k0 = a.k;
+    const float x0 = fm_fma<float>(s, a.g, a.e);
+    float x = x0;
+    bool three = false;
+    // the second term clearly out, or clearly in whichever of the first two
+    // comes first
+    bool in2 = b.k < x0;
+    bool ok = in2 ? b.k < x0 * (1.0f - kScreen) : b.k > x0 * (1.0f + kScreen);
+    const bool near01 = b.k * (1.0f - kScreen) <= a.k;
+    ok = ok && !(near01 && !(b.k * (1.0f + kScreen) < fm_min(x0, fm_fma<float>(s, b.g, b.e))));
+    if (in2) {
+        const float A = a.w + b.w, B = fm_fma<float>(a.w, a.e, b.w * b.e);
+        const float d01 = a.e - b.e, q01 = a.w * b.w * d01 * d01;
+        const float D = A * s2 - q01;
+        x = Fast<float>::div(B + Fast<float>::sqrt(fm_max(D, 0.0f)), A);
+        ok = ok && D >= A * s2 * (1.0f / 32.0f);
+        three = c.k < x;
+        ok = ok && (three ? c.k < x * (1.0f - kScreen) : c.k > x * (1.0f + kScreen));
+        const bool near12 = c.k * (1.0f - kScreen) <= b.k;
+        ok = ok && !(near12 && (b.e != b.k || c.e != c.k));
+        if (three) {
+            const float A3 = A + c.w, B3 = fm_fma<float>(c.w, c.e, B);
+            const float d02 = a.e - c.e, d12 = b.e - c.e;
+            const float D3 = A3 * s2 - (q01 + c.w * (a.w * d02 * d02 + b.w * d12 * d12));
+            x = Fast<float>::div(B3 + Fast<float>::sqrt(fm_max(D3, 0.0f)), A3);
+            ok = ok && D3 >= A3 * s2 * (1.0f / 32.0f);
+        }
+    }
+    r.x = x;
+    r.stands = ok;                                    // (false for NaN)
+    r.three = three && ok;
+    return r;
+}
+
+// The double-precision causal solve of one octant: terms in axis order, dt
+// the keys, dd = t1 - t2 where the axis is second order (o2), h and w the
+// spacings; three: all three terms are known to enter.  fm_update's
+// operations in its order.
+FM_HD double fm_octant(double s, const double dt[3], const double dd[3], unsigned o2, const Spacing<double> &sp,
+                       bool three)
+{
+    double e[3], w[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const bool o = (o2 >> a) & 1u;
+        e[a] = o ? fm_fma<double>(dd[a], 1.0 / 3.0, dt[a]) : dt[a];
+        w[a] = o ? sp.w[a] * 2.25 : sp.w[a];
+    }
+    // the lateral pair in order, then the radial term inserted (ties keep the
+    // order r, theta, phi)
+    const bool p = fm_less(dt[2], dt[1]);
+    const double kA = p ? dt[2] : dt[1], eA = p ? e[2] : e[1], wA = p ? w[2] : w[1];
+    const double kB = p ? dt[1] : dt[2], eB = p ? e[1] : e[2], wB = p ? w[1] : w[2];
+    const bool p1 = fm_less(kA, dt[0]);
+    const double e0 = p1 ? eA : e[0], w0 = p1 ? wA : w[0];
+    const double kM = p1 ? dt[0] : kA, eM = p1 ? e[0] : eA, wM = p1 ? w[0] : wA;
+    const bool p2 = fm_less(kB, kM);
+    const double k1 = p2 ? kB : kM, e1 = p2 ? eB : eM, w1 = p2 ? wB : wM;
+    const double k2 = p2 ? kM : kB, e2 = p2 ? eM : eB, w2 = p2 ? wM : wB;
+    // the first term's axis
+    const double hf = p1 ? (p ? sp.h[2] : sp.h[1]) : sp.h[0];
+    const bool of = ((p1 ? (p ? o2 >> 2 : o2 >> 1) : o2) & 1u) != 0;
+    double x = fm_fma<double>(s, of ? hf * (2.0 / 3.0) : hf, e0);
+    if (three || fm_less(k1, x)) {
+        const double s2 = s * s;
+        double a = w0 + w1;
+        const double we0 = w0 * e0, we1 = w1 * e1;
+        double b = we0 + we1;
+        double c = fm_fma<double>(we0, e0, fm_fma<double>(we1, e1, -s2));
+        if (!three) {
+            const double disc = fm_fma<double>(b, b, -(a * c));
+            x = (b + Fast<double>::sqrt(disc > 0.0 ? disc : 0.0)) / a;
+            three = fm_less(k2, x);
+        }
+        if (three) {
+            const double we2 = w2 * e2;
+            a += w2;
+            b += we2;
+            c = fm_fma<double>(we2, e2, c);
+            const double disc = fm_fma<double>(b, b, -(a * c));
+            x = (b + Fast<double>::sqrt(disc > 0.0 ? disc : 0.0)) / a;
+        }
+    }
+    return x;
+}
+
+template <>
+FM_HD double fm_update<double>(double s, const double t1[6], const double t2[6], unsigned inb,
+                               const Spacing<double> &sp, int order2)
+{
+    const double INF = Lim<double>::inf();
+    double tmin = INF;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) tmin = fm_less(t1[d], tmin) ? t1[d] : tmin;
+    if (!fm_less(tmin, INF)) return INF;
+    float hf[3], wf[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        hf[a] = fm_narrow(sp.h[a]);
+        wf[a] = fm_narrow(sp.w[a]);
+    }
+    const float sf = fm_narrow(s), s2f = sf * sf;
+    double dt[6], dd[6];
+    unsigned o2 = 0;
+    ScreenTerm t[6];
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+        const int a = d >> 1;
+        const bool o = order2 && fm_less(t2[d], t1[d]);
+        dt[d] = t1[d] - tmin;
+        dd[d] = o ? t1[d] - t2[d] : 0.0;
+        o2 |= o ? 1u << d : 0u;
+        t[d].k = fm_narrow(dt[d]);
+        t[d].e = o ? fm_fma<float>(fm_narrow(dd[d]), 1.0f / 3.0f, t[d].k) : t[d].k;
+        t[d].g = o ? hf[a] * (2.0f / 3.0f) : hf[a];
+        t[d].w = o ? wf[a] * 2.25f : wf[a];
+    }
+    // octant q: bit 0 the radial side, bit 1 theta, bit 2 phi
+    float lo[8];           // least value the octant can have, as far as the screen tells
+    unsigned three = 0;
+    float m = Lim<float>::inf();
+#pragma unroll
+    for (int lat = 0; lat < 4; ++lat) {
+        ScreenTerm a = t[2 + (lat & 1)], b = t[4 + (lat >> 1)];
+        fm_screen_swap(a, b);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int q = r | (lat << 1);
+            const unsigned om = (1u << r) | (4u << (lat & 1)) | (16u << (lat >> 1));
+            ScreenTerm x = t[r], y = a, z = b;
+            fm_screen_swap(x, y);
+            fm_screen_swap(y, z);
+            const Screened v = fm_screen(sf, s2f, x, y, z);
+            const bool in = (inb & om) == om;
+            lo[q] = in ? (v.stands ? v.x : v.k0) : Lim<float>::inf();
+            m = in && v.stands ? fm_min(m, v.x) : m;
+            three |= v.three ? 1u << q : 0u;
+        }
+    }
+    // (an octant outside the grid, or with no neighbour set, has lo = +inf)
+    const float cut = m * (1.0f + 2.0f * kScreen);
+    unsigned need = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) need |= lo[q] <= cut && lo[q] < Lim<float>::inf() ? 1u << q : 0u;
+    double best = INF;
+    while (need) {
+        const unsigned bit = need & (0u - need);
+        need ^= bit;
+        const bool r = (bit & 0xaau) != 0, x = (bit & 0xccu) != 0, z = (bit & 0xf0u) != 0;
+        const double kt[3] = {r ? dt[1] : dt[0], x ? dt[3] : dt[2], z ? dt[5] : dt[4]};
+        const double kd[3] = {r ? dd[1] : dd[0], x ? dd[3] : dd[2], z ? dd[5] : dd[4]};
+        const unsigned oo = ((o2 >> (r ? 1 : 0)) & 1u) | (((o2 >> (x ? 3 : 2)) & 1u) << 1) |
+                            (((o2 >> (z ? 5 : 4)) & 1u) << 2);
+        const double v = fm_octant(s, kt, kd, oo, sp, (three & bit) != 0);
+        best = fm_less(v, best) ? v : best;
+    }
+    return tmin + best;
+}
+
+// The upstream-only update, screened likewise over its seven subsets (bit 0
+// down, bit 1 theta, bit 2 phi).
+template <>
+FM_HD double fm_update_upstream<double>(double s, double tD, double tD2, double tX, double tX2, double tZ, double tZ2,
+                                        bool inD, bool inU, bool inXu, bool inXd, bool inZu, bool inZd,
+                                        const Spacing<double> &sp, int order2)
+{
+    const double INF = Lim<double>::inf();
+    const float INFF = Lim<float>::inf();
+    double tmin = fm_less(tX, tD) ? tX : tD;
+    tmin = fm_less(tZ, tmin) ? tZ : tmin;
+    if (!fm_less(tmin, INF)) return INF;
+    const double t1[3] = {tD, tX, tZ}, t2[3] = {tD2, tX2, tZ2};
+    const float sf = fm_narrow(s), s2f = sf * sf;
+    double dt[3], dd[3];
+    unsigned o2 = 0;
+    ScreenTerm t[3];
+    float x1[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const bool o = order2 && fm_less(t2[a], t1[a]);
+        dt[a] = t1[a] - tmin;
+        dd[a] = o ? t1[a] - t2[a] : 0.0;
+        o2 |= o ? 1u << a : 0u;
+        const float h = fm_narrow(sp.h[a]), w = fm_narrow(sp.w[a]);
+        t[a].k = fm_narrow(dt[a]);
+        t[a].e = o ? fm_fma<float>(fm_narrow(dd[a]), 1.0f / 3.0f, t[a].k) : t[a].k;
+        t[a].g = o ? h * (2.0f / 3.0f) : h;
+        t[a].w = o ? w * 2.25f : w;
+        x1[a] = fm_fma<float>(sf, t[a].g, t[a].e);
+    }
+    float lo[7];
+    unsigned three = 0;
+    float m = INFF;
+    // singles stand as they are
+    const bool c1[3] = {inD && inXd && inZd, inU && inXu && inZd, inU && inXd && inZu};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = c1[a] ? x1[a] : INFF;
+        m = fm_min(m, lo[a]);
+    }
+    const ScreenTerm none = {INFF, INFF, 1.0f, 1.0f};
+    const bool c2[4] = {inD && inXu && inZd, inD && inXd && inZu, inU && inXu && inZu, inD && inXu && inZu};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        // DX, DZ, XZ, DXZ
+        ScreenTerm x = t[j == 2 ? 1 : 0], y = t[j == 0 || j == 3 ? 1 : 2], z = j == 3 ? t[2] : none;
+        if (j == 3) fm_screen_swap(y, z);
+        fm_screen_swap(x, y);
+        if (j == 3) fm_screen_swap(y, z);
+        const Screened v = fm_screen(sf, s2f, x, y, z);
+        lo[3 + j] = c2[j] ? (v.stands ? v.x : v.k0) : INFF;
+        m = c2[j] && v.stands ? fm_min(m, v.x) : m;
+        if (j == 3 && v.three) three = 1;
+    }
+    const float cut = m * (1.0f + 2.0f * kScreen);
+    unsigned need = 0;
+#pragma unroll
+    for (int j = 0; j < 7; ++j) need |= lo[j] <= cut && lo[j] < INFF ? 1u << j : 0u;
+    double best = INF;
+    while (need) {
+        const unsigned bit = need & (0u - need);
+        need ^= bit;
+        // D in 0, 3, 4, 6; X in 1, 3, 5, 6; Z in 2, 4, 5, 6
+        const double kt[3] = {(bit & 0x59u) ? dt[0] : INF, (bit & 0x6au) ? dt[1] : INF, (bit & 0x74u) ? dt[2] : INF};
+        const double v = fm_octant(s, kt, dd, o2, sp, bit == 0x40u && three);
+        best = fm_less(v, best) ? v : best;
+    }
+    return tmin + best;
+}
+
 }  // namespace fm3dt
