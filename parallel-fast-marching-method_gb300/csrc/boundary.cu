@@ -9,6 +9,7 @@
 // Compiled without FMA contraction (plane-wave frames match the oracle's
 // double-precision formula bit for bit).
 #include <cfloat>
+#include <cstring>
 
 #include "internal.h"
 
@@ -40,7 +41,7 @@ __global__ void planewave_kernel(Geom g, PlaneWaveGeom pg, int nev, const double
 // (fixed nodes and their values) of the event's field.
 template <typename R>
 __global__ void finalize_kernel(Geom g, const double *__restrict__ frames, R *__restrict__ T,
-                                uint8_t *__restrict__ frozen, double *__restrict__ base, int offset_mode)
+                                uint8_t *__restrict__ frozen, double *__restrict__ base, int offset_mode, R unset)
 {
     const int e = blockIdx.x;
     const long long nb = (long long)g.nnx * g.nnz;
@@ -69,7 +70,7 @@ __global__ void finalize_kernel(Geom g, const double *__restrict__ frames, R *__
         const double v = fr[q];
         const bool fix = v > 0.0;                       // F:6932-6936
         fz[q] = fix ? 1 : 0;
-        bottom[q] = fix ? (R)(v - b) : (R)INFINITY;
+        bottom[q] = fix ? (R)(v - b) : unset;
     }
 }
 
@@ -77,17 +78,21 @@ __global__ void finalize_kernel(Geom g, const double *__restrict__ frames, R *__
 // boundary frame (sign of its summed theta and phi differences over pairs of
 // fixed nodes), which orders the solver's sweep.  bit 0: times grow with
 // theta (sweep +theta), bit 1: times grow with phi; bits 2 and 3: theta /
-// phi is a near tie (sweep it both ways).
+// phi is a near tie (sweep it both ways); bit 4: some nodes have no time.
 __global__ void directions_kernel(Geom g, const double *__restrict__ frames, int *__restrict__ dir, double tie_ratio)
 {
     const int e = blockIdx.x;
     const long long nb = (long long)g.nnx * g.nnz;
     const double *fr = frames + (size_t)e * nb;
     double sx = 0.0, sz = 0.0;
+    bool hole = false;
     for (long long q = threadIdx.x; q < nb; q += blockDim.x) {
         const int iz = (int)(q % g.nnz), ix = (int)(q / g.nnz);
         const double v = fr[q];
-        if (!(v > 0.0)) continue;
+        if (!(v > 0.0)) {
+            hole = true;
+            continue;
+        }
         if (ix + 1 < g.nnx && fr[q + g.nnz] > 0.0) sx += fr[q + g.nnz] - v;
         if (iz + 1 < g.nnz && fr[q + 1] > 0.0) sz += fr[q + 1] - v;
     }
@@ -97,7 +102,7 @@ __global__ void directions_kernel(Geom g, const double *__restrict__ frames, int
         sz += __shfl_xor_sync(0xffffffffu, sz, o);
     }
     if ((threadIdx.x & 31) == 0) { rx[threadIdx.x >> 5] = sx; rz[threadIdx.x >> 5] = sz; }
-    __syncthreads();
+    const bool holes = __syncthreads_or(hole) != 0;
     if (threadIdx.x == 0) {
         double ax = 0.0, az = 0.0;
         for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) { ax += rx[w]; az += rz[w]; }
@@ -106,7 +111,8 @@ __global__ void directions_kernel(Geom g, const double *__restrict__ frames, int
         // phi direction is ambiguous under heterogeneity and sweeps with that
         // direction reversed are worth their cost
         const double mx = fabs(ax), mz = fabs(az);
-        dir[e] = (ax >= 0.0 ? 1 : 0) | (az >= 0.0 ? 2 : 0) | (mx < tie_ratio * mz ? 4 : 0) | (mz < tie_ratio * mx ? 8 : 0);
+        dir[e] = (ax >= 0.0 ? 1 : 0) | (az >= 0.0 ? 2 : 0) | (mx < tie_ratio * mz ? 4 : 0) |
+                 (mz < tie_ratio * mx ? 8 : 0) | (holes ? 16 : 0);
     }
 }
 
@@ -164,12 +170,18 @@ void launch_planewave_frames(const Geom &g, const PlaneWaveGeom &pg, int nev, co
 }
 
 void launch_finalize_frames(const Geom &g, int nev, int prec, const double *frames, void *T, uint8_t *frozen,
-                            double *base, cudaStream_t st)
+                            double *base, bool unwritten, cudaStream_t st)
 {
+    double u64 = INFINITY;
+    float u32 = INFINITY;
+    if (unwritten) {
+        memset(&u64, 0xff, sizeof u64);
+        memset(&u32, 0xff, sizeof u32);
+    }
     if (prec == FM3DT_FP64)
-        finalize_kernel<double><<<nev, 512, 0, st>>>(g, frames, (double *)T, frozen, base, 0);
+        finalize_kernel<double><<<nev, 512, 0, st>>>(g, frames, (double *)T, frozen, base, 0, u64);
     else
-        finalize_kernel<float><<<nev, 512, 0, st>>>(g, frames, (float *)T, frozen, base, 1);
+        finalize_kernel<float><<<nev, 512, 0, st>>>(g, frames, (float *)T, frozen, base, 1, u32);
 }
 
 void launch_sweep_directions(const Geom &g, int nev, const double *frames, int *dir, double tie_ratio,

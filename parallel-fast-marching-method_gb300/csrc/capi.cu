@@ -322,8 +322,6 @@ const CUtensorMap *field_tensor_map(fm3dt_ctx *ctx, int shape)
 //                          of their single sweep fails
 //   FM_OVERLAP_MAIN        the near-tie events' main sweep on stream2 too, ahead of
 //                          their extra sweeps, beside the other events' main sweep
-//   FM_FRESH_SWEEP         main sweeps from the unset field with upstream-only node
-//                          updates (the same values as the full update there)
 //   FM_TIE_QUEUE           the near-tie events' last extra sweep queues the tiles
 //                          it changes for their first round, which then takes
 //                          those tiles instead of every tile
@@ -335,12 +333,7 @@ const CUtensorMap *field_tensor_map(fm3dt_ctx *ctx, int shape)
 #ifndef FM_TIE_SKIP
 #define FM_TIE_SKIP 1
 #endif
-//   FM_TIES_FIRST          in a two-part solve the other events' main sweep waits
-//                          for the near-tie events' one
-#ifndef FM_TIES_FIRST
-#define FM_TIES_FIRST 0
-#endif
-//   FM_SWEEP_FLOW          a streaming sweep pass as one launch whose items start
+//   FM_SWEEP_FLOW          a tracked extra sweep as one launch whose items start
 //                          when their upstream neighbours are done (instead of
 //                          one launch per hyperplane)
 #ifndef FM_SWEEP_FLOW
@@ -350,10 +343,6 @@ const CUtensorMap *field_tensor_map(fm3dt_ctx *ctx, int shape)
 #ifndef FM_FLOW_FIRST
 #define FM_FLOW_FIRST 1
 #endif
-//   FM_FLOW_TIE_MAIN       ... and the near-tie events' main sweep (stream2)
-#ifndef FM_FLOW_TIE_MAIN
-#define FM_FLOW_TIE_MAIN 0
-#endif
 //   FM_FLOW_SHARE_FIRST    percent of the resident slots a one-launch pass on stream2
 //   FM_FLOW_SHARE          takes: the chain's first tracked sweep (beside the other part's
 //                          certification), the later ones
@@ -362,9 +351,6 @@ const CUtensorMap *field_tensor_map(fm3dt_ctx *ctx, int shape)
 #endif
 #ifndef FM_FLOW_SHARE
 #define FM_FLOW_SHARE 75
-#endif
-#ifndef FM_FRESH_SWEEP
-#define FM_FRESH_SWEEP 1
 #endif
 #ifndef FM_ROUND0_PER_TILE
 #define FM_ROUND0_PER_TILE 1
@@ -431,9 +417,16 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), s));
     const bool do_sweep = ctx->sweep && mode == kFrames;
 
+    const bool streaming = ctx->sweep_shape >= kNumShapes;
     if (mode == kFrames) {
-        launch_fill_inf(ctx->d_T, (size_t)nev * ctx->N, ctx->prec, s);
-        launch_finalize_frames(g, nev, ctx->prec, ctx->d_frames, ctx->d_T, ctx->d_frozen, ctx->d_base, s);
+        // (the streaming main sweep writes every node, and waits for nodes
+        // that still hold ones)
+        const bool front = do_sweep && streaming;
+        if (front)
+            CK(cudaMemsetAsync(ctx->d_T, 0xff, (size_t)nev * ctx->N * rsize(ctx->prec), s));
+        else
+            launch_fill_inf(ctx->d_T, (size_t)nev * ctx->N, ctx->prec, s);
+        launch_finalize_frames(g, nev, ctx->prec, ctx->d_frames, ctx->d_T, ctx->d_frozen, ctx->d_base, front, s);
         launch_sweep_directions(g, nev, ctx->d_frames, ctx->d_dir, ctx->tie_ratio, s);
         ctx->launches += 3;
         CKL();
@@ -472,30 +465,76 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     int64_t sweep_nodes = 0;      // nodes visited by all sweep passes
     int64_t interval_nodes = 0;   // ... by the passes inside the sweep interval
     bool verified = false;
-    const bool streaming = ctx->sweep_shape >= kNumShapes;
     const int sidx = streaming ? ctx->sweep_shape - kNumShapes : 0;
     const int nbx = (g.nnx + kStreamShapes[sidx].sx - 1) / kStreamShapes[sidx].sx;
     const int nbz = (g.nnz + kStreamShapes[sidx].sz - 1) / kStreamShapes[sidx].sz;
-    // resident one-warp CTAs of the streaming sweep (the main sweep's form and
-    // the general form differ in registers)
-    auto stream_grid = [&](bool fresh, bool flow = false) {
-        return streaming ? std::max(1, ctx->prec == FM3DT_FP64 ? occupancy_stream_f64(sidx, fresh, flow)
-                                                               : occupancy_stream_f32(sidx, fresh, flow)) * sm_count()
+    // resident one-warp CTAs of the streaming sweep
+    auto stream_grid = [&](bool flow) {
+        return streaming ? std::max(1, ctx->prec == FM3DT_FP64 ? occupancy_stream_f64(sidx, flow)
+                                                               : occupancy_stream_f32(sidx, flow)) * sm_count()
                          : 1;
+    };
+    // The main sweep of nitems events (events == null: all), one launch.  The
+    // events of a group are swept side by side: as many as fill the resident
+    // warps one and a half times with the blocks that can be under way at
+    // once (a block trails those upstream by ~14 steps, so an event has
+    // nnr / 14 hyperplanes of blocks under way), no more, so that the halo
+    // columns are still in L2 when the next hyperplane reads them.
+    auto front_pass = [&](int nitems, const int *events, cudaStream_t st) -> int {
+        sweep_nodes += (int64_t)nitems * (int64_t)ctx->N;
+        const fm3dt_ctx::Planes *P = nullptr;
+        const int rc = ensure_block_planes(ctx, ctx->sweep_shape, 1, &P);
+        if (rc) return rc;
+        const int occ = ctx->prec == FM3DT_FP64 ? occupancy_front_f64(sidx) : occupancy_front_f32(sidx);
+        const double slots = (double)std::max(1, occ) * sm_count();
+        const int nblocks = nbx * nbz, planes = nbx + nbz - 1;
+        const double under_way = (double)nblocks / planes * std::min(planes, g.nnr / 14 + 1);
+        const int group = (int)std::min<double>(nitems, std::ceil(1.5 * slots / under_way));
+        const int si = st == ctx->stream2 ? 1 : 0;
+        CK(cudaMemsetAsync(ctx->d_next + si, 0, sizeof(unsigned), st));
+        auto fill = [&](auto &a) {
+            a.blocks = P->d_tiles;
+            a.nblocks = nblocks;
+            a.dir = ctx->d_dir;
+            a.events = events;
+            a.nev = nitems;
+            a.group = group;
+            a.nbx = nbx; a.nbz = nbz;
+            a.count = (unsigned)nblocks * (unsigned)nitems;
+            a.next = ctx->d_next + si;
+            // (all blocks resident at once: bound by the critical path, see
+            // front.cuh for both sides measured)
+            a.skew = a.count <= slots;
+            a.err = ctx->d_err;
+        };
+        if (ctx->prec == FM3DT_FP64) {
+            FrontArgs<double> a{};
+            a.f = f64;
+            fill(a);
+            launch_front_f64(sidx, a, st);
+        } else {
+            FrontArgs<float> a{};
+            a.f = f32;
+            fill(a);
+            launch_front_f32(sidx, a, st);
+        }
+        CKL();
+        sweep_launches += 1;
+        ctx->launches += 1;
+        return FM3DT_OK;
     };
     // One streaming sweep of nitems events (events == null: all), lateral
     // directions flipped by `flip`; with `flag`, changed nodes queue their
-    // tiles (and face neighbours) on list/count for the rounds.  `fresh`: the
-    // events' main sweep, from their unset fields (upstream-only updates).
+    // tiles (and face neighbours) on list/count for the rounds.
     // `recurs`: a pass that recurs from solve to solve (kept as a graph).
     // `act`: the item activity of a chain of sweeps (this sweep's, the
     // previous one's or null), see StreamArgs.
     auto stream_pass = [&](int nitems, const int *events, int flip, int nseg, int *flag, int *list,
-                           int *count, cudaStream_t st, bool fresh, bool recurs,
+                           int *count, cudaStream_t st, bool recurs,
                            unsigned *act_cur = nullptr, const unsigned *act_prev = nullptr,
                            unsigned long long *act_items = nullptr) -> int {
         sweep_nodes += (int64_t)nitems * (int64_t)ctx->N;
-        const int sgrid = stream_grid(fresh);
+        const int sgrid = stream_grid(false);
         if (nseg <= 0) nseg = stream_segments(ctx, nitems, nbx, nbz, sgrid, kStreamShapes[sidx].sx + kStreamShapes[sidx].sz - 2);
         nseg = std::min(nseg, g.nnr);
         // (no empty segment: 130 layers in 16 segments of 9 fill only 15; an
@@ -507,7 +546,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         if (rc) return rc;
         const auto &P = *PP;
         // (items of one layer or column would miss a 2-deep neighbour)
-        const bool track = !fresh && act_cur && seg_len >= 2 && kStreamShapes[sidx].sx >= 2;
+        const bool track = act_cur && seg_len >= 2 && kStreamShapes[sidx].sx >= 2;
         // One launch for the whole pass (FM_SWEEP_FLOW): items start as their
         // upstream neighbours finish, with a done flag per item and a queue
         // counter of the pass's stream, both zeroed ahead of the launch.  For
@@ -516,8 +555,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         // every item keep one launch per hyperplane, which shares the GPU with
         // the other stream's work (a one-launch pass holds every SM slot).
         const int si = st == ctx->stream2 ? 1 : 0;
-        const bool flow = FM_SWEEP_FLOW && streaming &&
-                          ((track && (act_prev != nullptr || FM_FLOW_FIRST)) || (fresh && si == 1 && FM_FLOW_TIE_MAIN));
+        const bool flow = FM_SWEEP_FLOW && streaming && track && (act_prev != nullptr || FM_FLOW_FIRST);
         const int nblocks = P.off.empty() ? 0 : P.off.back() + P.cnt.back();
         const size_t done_n = (size_t)nitems * (size_t)((g.nnr + seg_len - 1) / seg_len) * (size_t)nbx * (size_t)nbz;
         if (flow && done_n * sizeof(unsigned) > ctx->done_bytes[si]) {
@@ -531,7 +569,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         // (on stream2, beside the other part's work, a share of the resident
         // slots: a one-launch pass holds its slots to the end)
         const int fgrid = flow ? (int)std::min<long long>((long long)nblocks * nitems,
-                                                          std::max(1, stream_grid(fresh, true) *
+                                                          std::max(1, stream_grid(true) *
                                                                           (si ? (act_prev ? FM_FLOW_SHARE
                                                                                           : FM_FLOW_SHARE_FIRST)
                                                               : 100) / 100))
@@ -560,7 +598,6 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
                     a.dir = ctx->d_dir; a.nev = nitems; a.nbx = nbx; a.nbz = nbz;
                     a.events = events;
                     a.flip = flip;
-                    a.fresh = fresh ? 1 : 0;
                     a.seg_len = seg_len;
                     a.flag = flag;
                     a.list = list; a.count = count;
@@ -597,7 +634,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         bool launched = false;
         if (FM_SWEEP_GRAPHS && recurs && !ctx->sweep_graph_off) {
             const long long key[fm3dt_ctx::kSweepKey] = {ctx->prec, sidx, nitems, (long long)(intptr_t)events, flip,
-                                                         nseg, fresh ? 1 : 0, (long long)(intptr_t)st, ctx->shape,
+                                                         nseg, (long long)(intptr_t)st, ctx->shape,
                                                          (long long)(intptr_t)flag, (long long)(intptr_t)list,
                                                          (long long)(intptr_t)count, (long long)(intptr_t)act_cur,
                                                          (long long)(intptr_t)act_prev, (long long)(intptr_t)act_items,
@@ -658,8 +695,19 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         // sweeps, reversed and then forward
         CK(cudaMemcpyAsync(ctx->h_dir, ctx->d_dir, nev * sizeof(int), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        for (int e = 0; e < nev; ++e)
+        bool holes = false;
+        for (int e = 0; e < nev; ++e) {
             (ctx->h_dir[e] & 12 ? ties : others).push_back(e);
+            holes = holes || (ctx->h_dir[e] & 16);
+        }
+        if (holes) {
+            if (ctx->prec == FM3DT_FP64)
+                launch_holes_f64(f64, nev, s);
+            else
+                launch_holes_f32(f32, nev, s);
+            ctx->launches += 1;
+            CKL();
+        }
         // (only for large batches: with a few events the first round is short,
         // and contexts that solve side by side, as a service runs them, lose
         // more to the priority stream than they gain)
@@ -720,11 +768,13 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
                 (pass == 2 && !ctx->verify))
                 continue;
             const int nitems = pass == 1 ? (int)ties.size() : nev;
-            const int rc = stream_pass(nitems, pass == 1 ? ctx->d_events : nullptr, pl.flip,
-                                       pass == 1 ? ctx->tie_segments : ctx->sweep_segments,
-                                       pl.queue ? ctx->d_flag : nullptr, ctx->d_list[0], ctx->d_count[0], s,
-                                       pass == 0 && FM_FRESH_SWEEP, pass != 2, pass == 1 ? act_cur(pl.k) : nullptr,
-                                       pass == 1 ? act_prev(pl.k) : nullptr, pass == 1 ? act_items(pl.k) : nullptr);
+            const int rc = pass == 0 ? front_pass(nev, nullptr, s)
+                                     : stream_pass(nitems, pass == 1 ? ctx->d_events : nullptr, pl.flip,
+                                                   pass == 1 ? ctx->tie_segments : ctx->sweep_segments,
+                                                   pl.queue ? ctx->d_flag : nullptr, ctx->d_list[0], ctx->d_count[0], s,
+                                                   pass != 2, pass == 1 ? act_cur(pl.k) : nullptr,
+                                                   pass == 1 ? act_prev(pl.k) : nullptr,
+                                                   pass == 1 ? act_items(pl.k) : nullptr);
             if (rc) return rc;
         }
         CKL();
@@ -908,7 +958,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         CK(cudaEventCreate(&r1));
         CK(cudaMemcpyAsync(ev_buf, busy.data(), busy.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         CK(cudaEventRecord(r0, st));
-        const int rc = stream_pass((int)busy.size(), ev_buf, 0, 0, ctx->d_flag, list, count, st, false, false);
+        const int rc = stream_pass((int)busy.size(), ev_buf, 0, 0, ctx->d_flag, list, count, st, false);
         if (rc) return rc;
         interval_nodes += (int64_t)busy.size() * (int64_t)ctx->N;
         CK(cudaEventRecord(r1, st));
@@ -1065,19 +1115,10 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         CK(cudaStreamWaitEvent(s2, fork, 0));
         if (FM_OVERLAP_MAIN) {
             // each part's main sweep: the near-tie events' on stream2 ahead of
-            // their extra sweeps, the others' on the context stream -- after
-            // the near-tie events' (FM_TIES_FIRST), which then has the GPU to
-            // itself and starts the longer chain sooner, the others' main
-            // sweep filling the gaps of its extra sweeps
-            int rc = stream_pass((int)ties.size(), ctx->d_events, 0, ctx->tie_segments, nullptr, ctx->d_list[0],
-                                 ctx->d_count[0], s2, FM_FRESH_SWEEP, true);
+            // their extra sweeps, the others' on the context stream
+            int rc = front_pass((int)ties.size(), ctx->d_events, s2);
             if (rc) return rc;
-            if (FM_TIES_FIRST) {
-                CK(cudaEventRecord(pe[0], s2));
-                CK(cudaStreamWaitEvent(s, pe[0], 0));
-            }
-            rc = stream_pass((int)others.size(), ctx->d_events_b, 0, ctx->sweep_segments, nullptr, ctx->d_list[0],
-                             ctx->d_count[0], s, FM_FRESH_SWEEP, true);
+            rc = front_pass((int)others.size(), ctx->d_events_b, s);
             if (rc) return rc;
             interval_nodes += (int64_t)nev * (int64_t)ctx->N;
             CK(cudaEventRecord(sw1, s));
@@ -1097,7 +1138,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
             const bool q = tie_queue && k == ctx->tie_sweeps - 1;
             const int rc = stream_pass((int)ties.size(), ctx->d_events, (k & 1) ? 0 : 4,
                                        FM_OVERLAP_MAIN ? ctx->tie_segments : (ctx->tie_segments > 0 ? ctx->tie_segments : 2),
-                                       q ? ctx->d_flag : nullptr, ctx->d_list_b, ctx->d_count_b, s2, false, true,
+                                       q ? ctx->d_flag : nullptr, ctx->d_list_b, ctx->d_count_b, s2, true,
                                        act_cur(k), act_prev(k), act_items(k));
             if (rc) return rc;
         }
@@ -1214,7 +1255,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     if (kerr == 2) return fail(ctx, FM3DT_ECUDA, "a tile copy (TMA) destination was not 128-byte aligned");
     if (kerr & 4) return fail(ctx, FM3DT_ECUDA, "a tracked sweep met an activity slot out of range");
     if (kerr & 16)
-        return fail(ctx, FM3DT_ECUDA, "a one-launch sweep pass gave up waiting for an item's upstream neighbours");
+        return fail(ctx, FM3DT_ECUDA, "a sweep gave up waiting for upstream columns");
     if (kerr) return fail(ctx, FM3DT_ECUDA, "a tile copy (TMA) did not complete in time");
     if (!done) return fail(ctx, FM3DT_ENOCONV, "solver round limit reached before convergence");
     return FM3DT_OK;

@@ -106,7 +106,6 @@ struct StreamArgs {
     const int *events;          // the events swept (indices), or null for events 0..nev-1
     int nev;
     int flip;                   // bit 0 / 1: reverse theta / phi; bit 2: reverse each near-tie lateral direction
-    int fresh;                  // the main sweep from an unset field: upstream-only node updates
     int nbx, nbz;               // column blocks per axis
     int seg_len;                // layers per height segment
     // verification sweep: when flag is set, every node whose value changes
@@ -143,10 +142,35 @@ struct StreamArgs {
     unsigned *next;
 };
 
+// The main sweep (front.cuh): every listed event once, from a field filled
+// with ones above its boundary layer.
+template <typename R>
+struct FrontArgs {
+    FieldArgs<R> f;
+    const int *blocks;          // swept column blocks x' << 12 | z', by hyperplane
+    int nblocks;
+    const int *dir;             // [E] bit 0: sweep +theta, bit 1: sweep +phi
+    const int *events;          // the events swept (indices), or null for events 0..nev-1
+    int nev;
+    int group;                  // events swept together (blocks are taken group by group)
+    int nbx, nbz;               // column blocks per axis
+    unsigned count;             // nblocks * nev
+    int skew;                   // halo columns and values pass from lane to lane, not layer by layer
+    unsigned *next;             // blocks taken so far (zero at the start)
+    int *err;                   // bit 4 raised: a wait for an upstream block gave up
+};
+void launch_front_f32(int idx, const FrontArgs<float> &a, cudaStream_t st);
+void launch_front_f64(int idx, const FrontArgs<double> &a, cudaStream_t st);
+// start values of boundary nodes without a time, ahead of the main sweep
+void launch_holes_f32(const FieldArgs<float> &f, int nev, cudaStream_t st);
+void launch_holes_f64(const FieldArgs<double> &f, int nev, cudaStream_t st);
+int occupancy_front_f32(int idx);
+int occupancy_front_f64(int idx);
+
 void launch_stream_f32(int idx, int grid, const StreamArgs<float> &a, cudaStream_t st);
 void launch_stream_f64(int idx, int grid, const StreamArgs<double> &a, cudaStream_t st);
-int occupancy_stream_f32(int idx, bool fresh, bool flow = false);
-int occupancy_stream_f64(int idx, bool fresh, bool flow = false);
+int occupancy_stream_f32(int idx, bool flow);
+int occupancy_stream_f64(int idx, bool flow);
 
 // After a single sweep from an unset field: mark the nodes a recomputation
 // could change (certification bitmap) and queue their tiles (kCert).
@@ -192,8 +216,10 @@ void launch_gridder(const Geom &g, const double *velv, double *veln, void *s, in
 struct PlaneWaveGeom { double rb, thc, phc, rbs; };
 void launch_planewave_frames(const Geom &g, const PlaneWaveGeom &pg, int nev, const double *params,
                              double *frames, cudaStream_t st);
+// (unwritten: boundary nodes without a time get all ones, to be written by the
+// main sweep, instead of +inf)
 void launch_finalize_frames(const Geom &g, int nev, int prec, const double *frames, void *T,
-                            uint8_t *frozen, double *base, cudaStream_t st);
+                            uint8_t *frozen, double *base, bool unwritten, cudaStream_t st);
 void launch_fill_inf(void *T, size_t n, int prec, cudaStream_t st);
 // n doubles between device memory and the device mapping of page-locked host
 // memory (either way round), by a kernel
@@ -397,7 +423,7 @@ struct fm3dt_ctx {
     // count, event list, flip, height segments, form, stream, tile shape,
     // (flag mode) the flags and queue it writes, the activity it tracks and
     // (one-launch passes) its done flags
-    static constexpr int kSweepKey = 16;
+    static constexpr int kSweepKey = 15;
     static constexpr size_t kSweepGraphs = 24;
     struct SweepGraph { long long key[kSweepKey]; cudaGraphExec_t exec; };
     std::vector<SweepGraph> sweep_graphs;

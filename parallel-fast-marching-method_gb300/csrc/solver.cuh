@@ -491,7 +491,8 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
 // (about 1e-3 of the octant's largest term in single precision); octants
 // that take none are unchanged bit for bit; the earliest neighbour stays the
 // same, and the terms below B come first in every sort as before.  Nodes
-// that fail, and unreached nodes, go into the bitmap.
+// that fail, unreached nodes, and boundary nodes without a time (whose start
+// value may come from downstream neighbours) go into the bitmap.
 template <typename R>
 __global__ void __launch_bounds__(256, 4) certify_kernel(const CertifyArgs<R> a)
 {
@@ -561,6 +562,7 @@ __global__ void __launch_bounds__(256, 4) certify_kernel(const CertifyArgs<R> a)
                     // one outside the grid reads unset and passes
                     auto down_ok = [&](R t1, R t2) { return (t1 - tu) >= hi && !(f.order2 && t2 < t1); };
                     ok = ok && down_ok(v1, v0) && down_ok(txd, txd2) && down_ok(tzd, tzd2);
+                    if (gr == f.nnr - 1) ok = false;
                     // an upstream neighbour at or above lo must be first order
                     if (f.order2) {
                         if (gr < f.nnr - 1 && !((td - tu) < lo) && v4 < td) ok = false;

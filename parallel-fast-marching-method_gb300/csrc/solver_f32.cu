@@ -55,10 +55,38 @@ void launch_stream_f32(int idx, int grid, const StreamArgs<float> &a, cudaStream
 #undef C_
 }
 
-int occupancy_stream_f32(int idx, bool fresh, bool flow)
+int occupancy_stream_f32(int idx, bool flow)
 {
     int r = 0;
-#define C_(X, Z) r = StreamKernels<float, X, Z>::occ(fresh, flow)
+#define C_(X, Z) r = StreamKernels<float, X, Z>::occ(flow)
+    FM_STREAM_SWITCH(idx, C_)
+#undef C_
+    return r;
+}
+
+}  // namespace fm3dt
+
+// main sweep
+#include "front.cuh"
+
+namespace fm3dt {
+
+void launch_front_f32(int idx, const FrontArgs<float> &a, cudaStream_t st)
+{
+#define C_(X, Z) launch_front<float, X, Z>(a, st)
+    FM_STREAM_SWITCH(idx, C_)
+#undef C_
+}
+
+void launch_holes_f32(const FieldArgs<float> &f, int nev, cudaStream_t st)
+{
+    launch_holes<float>(f, nev, st);
+}
+
+int occupancy_front_f32(int idx)
+{
+    int r = 0;
+#define C_(X, Z) r = occupancy_front<float, X, Z>()
     FM_STREAM_SWITCH(idx, C_)
 #undef C_
     return r;

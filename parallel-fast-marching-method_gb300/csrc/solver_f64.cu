@@ -55,10 +55,38 @@ void launch_stream_f64(int idx, int grid, const StreamArgs<double> &a, cudaStrea
 #undef C_
 }
 
-int occupancy_stream_f64(int idx, bool fresh, bool flow)
+int occupancy_stream_f64(int idx, bool flow)
 {
     int r = 0;
-#define C_(X, Z) r = StreamKernels<double, X, Z>::occ(fresh, flow)
+#define C_(X, Z) r = StreamKernels<double, X, Z>::occ(flow)
+    FM_STREAM_SWITCH(idx, C_)
+#undef C_
+    return r;
+}
+
+}  // namespace fm3dt
+
+// main sweep
+#include "front.cuh"
+
+namespace fm3dt {
+
+void launch_front_f64(int idx, const FrontArgs<double> &a, cudaStream_t st)
+{
+#define C_(X, Z) launch_front<double, X, Z>(a, st)
+    FM_STREAM_SWITCH(idx, C_)
+#undef C_
+}
+
+void launch_holes_f64(const FieldArgs<double> &f, int nev, cudaStream_t st)
+{
+    launch_holes<double>(f, nev, st);
+}
+
+int occupancy_front_f64(int idx)
+{
+    int r = 0;
+#define C_(X, Z) r = occupancy_front<double, X, Z>()
     FM_STREAM_SWITCH(idx, C_)
 #undef C_
     return r;

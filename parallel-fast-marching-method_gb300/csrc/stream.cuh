@@ -1,5 +1,5 @@
-// stream.cuh -- streaming directional sweep (an alternative to the tile sweep
-// of solver.cuh).
+// stream.cuh -- streaming sweeps after the main one (front.cuh): the extra
+// sweeps of near-tie events, re-sweeps and the verifying sweep.
 //
 // One warp owns a block of SX x SZ (theta, phi) columns and streams through
 // one height segment of the grid (the whole height, or a few tens of layers
@@ -14,7 +14,7 @@
 // neighbours are in earlier launches.  Events whose lateral direction is a
 // near tie are swept twice more, with that direction reversed and then
 // forward again; events still changing on many tiles after a round are swept
-// again (flag mode: changed nodes queue their tiles).  The sweep is only a
+// again (flag mode: changed nodes queue their tiles).  A sweep is only a
 // good start for the rounds, which reach the same fixed point from
 // any start.
 #pragma once
@@ -215,18 +215,7 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
-// FRESH: the main sweep of a solve, from an unset field (every node except
-// the fixed bottom layer unset).  Each node above the bottom layer then sees
-// its downstream neighbours (up, and the lateral ones the sweep runs toward)
-// still unset -- later lanes of the block and later launches have not
-// written them, and the node's update must not take them -- so it is
-// computed by fm_update_upstream, which gives fm_update's value with those
-// neighbours unset from the three upstream ones alone.  (Items of the same
-// hyperplane may already have written a downstream neighbour in a halo
-// column; the upstream form leaves it out, as a sweep from an unset field
-// would, and the rounds reach the same fixed point either way.)  The bottom
-// layer keeps fm_update: fixed boundary nodes beside an unset one are set.
-template <typename R, int SX, int SZ, bool FRESH, bool FLOW>
+template <typename R, int SX, int SZ, bool FLOW>
 __device__ __forceinline__ void stream_sweep_body(const StreamArgs<R> &a)
 {
     static_assert(SX * SZ == 32, "one warp per column block");
@@ -322,7 +311,7 @@ __device__ __forceinline__ void stream_sweep_body(const StreamArgs<R> &a)
         }
         {
         // activity: the chunks that run
-        if (!FRESH && a.act_cur) {
+        if (a.act_cur) {
             const size_t aslot = slot;
             unsigned run = ~0u;
             if (a.act_prev) {
@@ -398,7 +387,7 @@ __device__ __forceinline__ void stream_sweep_body(const StreamArgs<R> &a)
             if (colv && rp + 1 >= lo && rp + 1 < hi) pnext = TL::params_global(f, f.nnr - 2 - rp, gx, gz);
             // (tracked sweeps: the step runs when a lane's node lies in a
             // chunk that can change)
-            if (!FRESH && a.act_cur &&
+            if (a.act_cur &&
                 !__any_sync(0xffffffffu, colv && rp >= lo && rp < hi && ((s_active >> ((rp - lo) >> a.act_shift)) & 1u))) {
                 // A quiet step.  The first step from here with a node in a
                 // chunk that can change (at step t the lanes hold layers
@@ -452,33 +441,22 @@ __device__ __forceinline__ void stream_sweep_body(const StreamArgs<R> &a)
                     const R *Lu2 = ring + ((rp + 2 + RING) & (RING - 1)) * LAYER;
                     const R *Ld1 = ring + ((rp - 1 + RING) & (RING - 1)) * LAYER;
                     const R *Ld2 = ring + ((rp - 2 + RING) & (RING - 1)) * LAYER;
-                    R v;
-                    if (FRESH && rp >= 1) {
-                        // upstream: down, and x-1 / z-1 when the sweep runs
-                        // toward +theta / +phi (else x+1 / z+1)
-                        const int ox = sx ? -LZ : LZ, oz = sz ? -1 : 1;
-                        const bool xlo = gx > 0, xhi = gx < f.nnx - 1, zlo = gz > 0, zhi = gz < f.nnz - 1;
-                        v = fm_update_upstream<R>(pcur.s, Ld1[c], Ld2[c], L0[c + ox], L0[c + 2 * ox], L0[c + oz],
-                                                  L0[c + 2 * oz], true, gr > 0, sx ? xlo : xhi, sx ? xhi : xlo,
-                                                  sz ? zlo : zhi, sz ? zhi : zlo, pcur.sp, f.order2);
-                    } else {
-                        R t1[6], t2[6];
-                        t1[0] = Lu1[c];       t2[0] = Lu2[c];          // r-1 (up)
-                        t1[1] = Ld1[c];       t2[1] = Ld2[c];          // r+1 (down)
-                        t1[2] = L0[c - LZ];   t2[2] = L0[c - 2 * LZ];
-                        t1[3] = L0[c + LZ];   t2[3] = L0[c + 2 * LZ];
-                        t1[4] = L0[c - 1];    t2[4] = L0[c - 2];
-                        t1[5] = L0[c + 1];    t2[5] = L0[c + 2];
-                        const unsigned inb = (gr > 0 ? 1u : 0u) | (gr < f.nnr - 1 ? 2u : 0u) | (gx > 0 ? 4u : 0u) |
-                                             (gx < f.nnx - 1 ? 8u : 0u) | (gz > 0 ? 16u : 0u) |
-                                             (gz < f.nnz - 1 ? 32u : 0u);
-                        v = fm_update<R>(pcur.s, t1, t2, inb, pcur.sp, f.order2);
-                    }
+                    R t1[6], t2[6];
+                    t1[0] = Lu1[c];       t2[0] = Lu2[c];          // r-1 (up)
+                    t1[1] = Ld1[c];       t2[1] = Ld2[c];          // r+1 (down)
+                    t1[2] = L0[c - LZ];   t2[2] = L0[c - 2 * LZ];
+                    t1[3] = L0[c + LZ];   t2[3] = L0[c + 2 * LZ];
+                    t1[4] = L0[c - 1];    t2[4] = L0[c - 2];
+                    t1[5] = L0[c + 1];    t2[5] = L0[c + 2];
+                    const unsigned inb = (gr > 0 ? 1u : 0u) | (gr < f.nnr - 1 ? 2u : 0u) | (gx > 0 ? 4u : 0u) |
+                                         (gx < f.nnx - 1 ? 8u : 0u) | (gz > 0 ? 16u : 0u) |
+                                         (gz < f.nnz - 1 ? 32u : 0u);
+                    const R v = fm_update<R>(pcur.s, t1, t2, inb, pcur.sp, f.order2);
                     const R old = L0[c];
                     if (fbits(v) != fbits(old)) {
                         ring[((rp + RING) & (RING - 1)) * LAYER + c] = v;
                         Te[((size_t)gr * f.nnx + gx) * f.nnz + gz] = v;
-                        if (!FRESH && a.act_cur) {
+                        if (a.act_cur) {
                             // this chunk changed; it and its neighbours can change further
                             const unsigned b = 1u << ((rp - lo) >> a.act_shift);
                             atomicOr(&s_changed, b);
@@ -490,7 +468,7 @@ __device__ __forceinline__ void stream_sweep_body(const StreamArgs<R> &a)
             }
             __syncwarp();
         }
-        if (!FRESH && a.act_cur && lane == 0 && s_aslot < a.act_n) a.act_cur[s_aslot] = s_changed;
+        if (a.act_cur && lane == 0 && s_aslot < a.act_n) a.act_cur[s_aslot] = s_changed;
         }
     item_done:
         if (FLOW) {
@@ -510,24 +488,23 @@ __device__ __forceinline__ void stream_sweep_body(const StreamArgs<R> &a)
 
 // The per-hyperplane form (one launch per hyperplane of a pass) and the
 // one-launch form, each with its own register budget: the one-launch form
-// holds its items' queue state, and is bounded to the resident CTAs of the
-// per-hyperplane form's main sweep.
+// holds its items' queue state.
 #ifndef FM_FLOW_BLOCKS_F32
 #define FM_FLOW_BLOCKS_F32 20
 #endif
 template <typename R> struct FlowBlocks { static constexpr int value = FM_FLOW_BLOCKS_F32; };
 template <> struct FlowBlocks<double> { static constexpr int value = 12; };
 
-template <typename R, int SX, int SZ, bool FRESH>
+template <typename R, int SX, int SZ>
 __global__ void __launch_bounds__(32) stream_sweep_kernel(StreamArgs<R> a)
 {
-    stream_sweep_body<R, SX, SZ, FRESH, false>(a);
+    stream_sweep_body<R, SX, SZ, false>(a);
 }
 
-template <typename R, int SX, int SZ, bool FRESH>
+template <typename R, int SX, int SZ>
 __global__ void __launch_bounds__(32, FlowBlocks<R>::value) stream_flow_kernel(StreamArgs<R> a)
 {
-    stream_sweep_body<R, SX, SZ, FRESH, true>(a);
+    stream_sweep_body<R, SX, SZ, true>(a);
 }
 
 template <typename R, int SX, int SZ>
@@ -535,35 +512,23 @@ struct StreamKernels {
     static void sweep(int grid, const StreamArgs<R> &a, cudaStream_t st)
     {
         if (a.flow) {
-            if (a.fresh)
-                stream_flow_kernel<R, SX, SZ, true><<<grid, 32, 0, st>>>(a);
-            else
-                stream_flow_kernel<R, SX, SZ, false><<<grid, 32, 0, st>>>(a);
+            stream_flow_kernel<R, SX, SZ><<<grid, 32, 0, st>>>(a);
             return;
         }
-        if (!a.fresh && a.act_cur && a.act_prev) {
+        if (a.act_cur && a.act_prev) {
             const long long items = (long long)a.hcount * a.nev;
             const int blocks = (int)std::min<long long>((items + 127) / 128, 4096);
             stream_activity_kernel<R><<<blocks, 128, 0, st>>>(a);
         }
-        if (a.fresh)
-            stream_sweep_kernel<R, SX, SZ, true><<<grid, 32, 0, st>>>(a);
-        else
-            stream_sweep_kernel<R, SX, SZ, false><<<grid, 32, 0, st>>>(a);
+        stream_sweep_kernel<R, SX, SZ><<<grid, 32, 0, st>>>(a);
     }
-    static int occ(bool fresh, bool flow)
+    static int occ(bool flow)
     {
         int nb = 0;
-        if (flow) {
-            if (fresh)
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stream_flow_kernel<R, SX, SZ, true>, 32, 0);
-            else
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stream_flow_kernel<R, SX, SZ, false>, 32, 0);
-        } else if (fresh) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stream_sweep_kernel<R, SX, SZ, true>, 32, 0);
-        } else {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stream_sweep_kernel<R, SX, SZ, false>, 32, 0);
-        }
+        if (flow)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stream_flow_kernel<R, SX, SZ>, 32, 0);
+        else
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stream_sweep_kernel<R, SX, SZ>, 32, 0);
         return nb;
     }
 };
