@@ -137,16 +137,25 @@ struct Tile {
     static __device__ __forceinline__ R update_with(const R *sm, int c, const FieldArgs<R> &a, int gr, int gx, int gz,
                                                     const Params &p)
     {
-        R t1[6], t2[6];
+        const unsigned inb = (gr > 0 ? 1u : 0u) | (gr < a.nnr - 1 ? 2u : 0u) | (gx > 0 ? 4u : 0u) |
+                             (gx < a.nnx - 1 ? 8u : 0u) | (gz > 0 ? 16u : 0u) | (gz < a.nnz - 1 ? 32u : 0u);
+        R t1[6], t2[6], v;
+        neighbours(sm, c, t1, t2);
+        if constexpr (sizeof(R) == 8) return fm_update<R>(p.s, t1, t2, inb, p.sp, a.order2);
+        if (fm_update_near<R>(p.s, t1, t2, inb, p.sp, a.order2, v)) return v;
+        // (read again rather than held in registers through the short form)
+        asm volatile("" ::: "memory");
+        neighbours(sm, c, t1, t2);
+        return fm_update_octants<R>(p.s, t1, t2, inb, p.sp, a.order2);
+    }
+    static __device__ __forceinline__ void neighbours(const R *sm, int c, R (&t1)[6], R (&t2)[6])
+    {
         t1[0] = sm[c - SR];     t2[0] = sm[c - 2 * SR];
         t1[1] = sm[c + SR];     t2[1] = sm[c + 2 * SR];
         t1[2] = sm[c - BZ];     t2[2] = sm[c - 2 * BZ];
         t1[3] = sm[c + BZ];     t2[3] = sm[c + 2 * BZ];
         t1[4] = sm[c - 1];      t2[4] = sm[c - 2];
         t1[5] = sm[c + 1];      t2[5] = sm[c + 2];
-        const unsigned inb = (gr > 0 ? 1u : 0u) | (gr < a.nnr - 1 ? 2u : 0u) | (gx > 0 ? 4u : 0u) |
-                             (gx < a.nnx - 1 ? 8u : 0u) | (gz > 0 ? 16u : 0u) | (gz < a.nnz - 1 ? 32u : 0u);
-        return fm_update<R>(p.s, t1, t2, inb, p.sp, a.order2);
     }
 
     // one node update (tile-local r, tx, tz) from shared memory; returns the
@@ -168,10 +177,12 @@ struct Tile {
 };
 
 // Resident 128-thread CTAs per SM that the register allocation must allow.
+// (Rounds in single precision: 6, 80 registers, since the short form of the
+// update; with 8 and 64 registers it spills.)
 // The kernels are issue-bound with long dependent chains, so occupancy pays
 // until registers spill.
 #ifndef FM_ROUND_MINB_F32
-#define FM_ROUND_MINB_F32 8
+#define FM_ROUND_MINB_F32 6
 #endif
 #ifndef FM_ROUND_MINB_F64
 #define FM_ROUND_MINB_F64 4

@@ -158,8 +158,11 @@ template <typename R> struct Spacing {
 // order, the same equation as the reference's (3T - 4 t1 + t2)/(2h) term),
 // relative to tmin, the earliest in-grid neighbour.  Every octant sorts its
 // three terms by t1 and adds them while t1 < T (the causal solve).
+//
+// This is the general form; fm_update below takes it only where its shorter
+// form does not hold.
 template <typename R>
-FM_HD R fm_update(R s, const R t1[6], const R t2[6], unsigned inb, const Spacing<R> &sp, int order2)
+FM_HD R fm_update_octants(R s, const R t1[6], const R t2[6], unsigned inb, const Spacing<R> &sp, int order2)
 {
     const R INF = Lim<R>::inf();
     // (a neighbour outside the grid holds +inf or NaN, which the hardware
@@ -282,30 +285,30 @@ FM_HD R fm_update(R s, const R t1[6], const R t2[6], unsigned inb, const Spacing
 // tD/tD2, tX/tX2, tZ/tZ2: upstream first and second neighbour values;
 // in*: whether each upstream (u) and downstream (d) neighbour lies inside the
 // grid (inD: r+1, inU: r-1).
+// The seven subsets' least value, relative to tmin (the least of the three
+// times): t1, t2 the three sides' first and second neighbour values (D, X, Z
+// above), n / f: whether each of these sides, and the opposite one, lies inside
+// the grid.
 template <typename R>
-FM_HD R fm_update_upstream(R s, R tD, R tD2, R tX, R tX2, R tZ, R tZ2, bool inD, bool inU, bool inXu, bool inXd,
-                           bool inZu, bool inZd, const Spacing<R> &sp, int order2)
+FM_HD R fm_subsets(R s, const R t1[3], const R t2[3], R tmin, bool n0, bool f0, bool n1, bool f1, bool n2, bool f2,
+                   const Spacing<R> &sp, int order2)
 {
     const R INF = Lim<R>::inf();
-    const R tmin = fm_min(fm_min(tD, tX), tZ);
     const R s2 = s * s;
     // (with an unset neighbour, or all of them, differences are +inf or NaN:
     // no comparison lets them in, and an unset tmin is selected at the end)
     R k[3], e[3], w[3], we[3], x1[3], q[3];
-    {
-        const R t1[3] = {tD, tX, tZ}, t2[3] = {tD2, tX2, tZ2};
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const bool o2 = order2 && (t2[a] < t1[a]);
-            const R dt = t1[a] - tmin;
-            k[a] = dt;
-            e[a] = o2 ? fm_fma<R>(t1[a] - t2[a], R(1.0 / 3.0), dt) : dt;
-            const R g = o2 ? sp.h[a] * R(2.0 / 3.0) : sp.h[a];
-            w[a] = o2 ? sp.w[a] * R(2.25) : sp.w[a];
-            x1[a] = fm_fma<R>(s, g, e[a]);        // the one-term solution
-            we[a] = w[a] * e[a];
-            q[a] = fm_fma<R>(we[a], e[a], -s2);
-        }
+    for (int a = 0; a < 3; ++a) {
+        const bool o2 = order2 && (t2[a] < t1[a]);
+        const R dt = t1[a] - tmin;
+        k[a] = dt;
+        e[a] = o2 ? fm_fma<R>(t1[a] - t2[a], R(1.0 / 3.0), dt) : dt;
+        const R g = o2 ? sp.h[a] * R(2.0 / 3.0) : sp.h[a];
+        w[a] = o2 ? sp.w[a] * R(2.25) : sp.w[a];
+        x1[a] = fm_fma<R>(s, g, e[a]);        // the one-term solution
+        we[a] = w[a] * e[a];
+        q[a] = fm_fma<R>(we[a], e[a], -s2);
     }
     // causal solves of the pairs DX, DZ, XZ (i before j in axis order, sorted
     // stably): the two-term step exactly as fm_update's
@@ -343,17 +346,83 @@ FM_HD R fm_update_upstream(R s, R tD, R tD2, R tX, R tX2, R tZ, R tZ2, bool inD,
     const R xt = on2 && kL < x2 ? x3 : x2;
     // subsets whose octant lies inside the grid (upstream side on the axes in
     // the subset, downstream side on the others).  (At the bottom layer, D
-    // unset and r-1 inside, inD may be passed as true: the octants with D then
+    // unset and r-1 inside, n0 may be passed as true: the octants with D then
     // give what those with r-1 give.)
     R best = INF;
-    best = inD && inXd && inZd ? fm_min(best, x1[0]) : best;
-    best = inU && inXu && inZd ? fm_min(best, x1[1]) : best;
-    best = inU && inXd && inZu ? fm_min(best, x1[2]) : best;
-    best = inD && inXu && inZd ? fm_min(best, xp[0]) : best;
-    best = inD && inXd && inZu ? fm_min(best, xp[1]) : best;
-    best = inU && inXu && inZu ? fm_min(best, xp[2]) : best;
-    best = inD && inXu && inZu ? fm_min(best, xt) : best;
+    best = n0 && f1 && f2 ? fm_min(best, x1[0]) : best;
+    best = f0 && n1 && f2 ? fm_min(best, x1[1]) : best;
+    best = f0 && f1 && n2 ? fm_min(best, x1[2]) : best;
+    best = n0 && n1 && f2 ? fm_min(best, xp[0]) : best;
+    best = n0 && f1 && n2 ? fm_min(best, xp[1]) : best;
+    best = f0 && n1 && n2 ? fm_min(best, xp[2]) : best;
+    best = n0 && n1 && n2 ? fm_min(best, xt) : best;
+    return best;
+}
+
+template <typename R>
+FM_HD R fm_update_upstream(R s, R tD, R tD2, R tX, R tX2, R tZ, R tZ2, bool inD, bool inU, bool inXu, bool inXd,
+                           bool inZu, bool inZd, const Spacing<R> &sp, int order2)
+{
+    const R INF = Lim<R>::inf();
+    const R t1[3] = {tD, tX, tZ}, t2[3] = {tD2, tX2, tZ2};
+    const R tmin = fm_min(fm_min(tD, tX), tZ);
+    const R best = fm_subsets<R>(s, t1, t2, tmin, inD, inU, inXu, inXd, inZu, inZd, sp, order2);
     return tmin < INF ? tmin + best : INF;
+}
+
+// The node update's short form (false: it does not hold).  On each axis the earlier neighbour is the near side, the
+// other the far side.  Where every far side is first order and its key at
+// least B (1 + kNear), B the least value of the near sides' seven subsets, and
+// no near side with a key of B (1 - kNear) or more is second order, the eight
+// octants' least value is B, bit for bit: adding a first-order causal term
+// with key k to an octant's solve gives a root above k (the quadratic is below
+// s^2 at k, or its vertex lies above k), so an octant that takes a far side
+// ends above B (1 + kNear) less the solve's rounding (at most ~7e-4 of it in
+// single precision, a discriminant near zero losing half its digits), and
+// one that takes none is the solve of its near sides, which is a subset's.
+// (An unset or outside far side is never taken.)  The seven subsets are four
+// quadratics in straight-line code, the octants up to sixteen behind
+// branches; in a sweep or a round nearly every node takes the short form.
+constexpr float kNear = 1.0f / 256.0f;
+
+template <typename R>
+FM_HD bool fm_update_near(R s, const R t1[6], const R t2[6], unsigned inb, const Spacing<R> &sp, int order2, R &out)
+{
+    const R INF = Lim<R>::inf();
+    R n1[3], n2[3], f1[3], f2[3];
+    bool nin[3], fin[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const bool ia = (inb >> (2 * a)) & 1u, ib = (inb >> (2 * a + 1)) & 1u;
+        const R ta = ia ? t1[2 * a] : INF, tb = ib ? t1[2 * a + 1] : INF;
+        const bool p = tb < ta;
+        n1[a] = p ? tb : ta;
+        f1[a] = p ? ta : tb;
+        n2[a] = p ? t2[2 * a + 1] : t2[2 * a];
+        f2[a] = p ? t2[2 * a] : t2[2 * a + 1];
+        nin[a] = p ? ib : ia;
+        fin[a] = p ? ia : ib;
+    }
+    const R tmin = fm_min(fm_min(n1[0], n1[1]), n1[2]);
+    out = INF;
+    if (!(tmin < INF)) return true;
+    const R best = fm_subsets<R>(s, n1, n2, tmin, nin[0], fin[0], nin[1], fin[1], nin[2], fin[2], sp, order2);
+    const R hi = fm_fma<R>(best, R(kNear), best), lo = fm_fma<R>(best, R(-kNear), best);
+    bool ok = best < INF;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        ok = ok && f1[a] - tmin >= hi && !(order2 && f2[a] < f1[a] && f1[a] < INF);
+        ok = ok && !(order2 && n2[a] < n1[a] && n1[a] - tmin >= lo && n1[a] < INF);
+    }
+    out = tmin + best;
+    return ok;
+}
+
+template <typename R>
+FM_HD R fm_update(R s, const R t1[6], const R t2[6], unsigned inb, const Spacing<R> &sp, int order2)
+{
+    R v;
+    return fm_update_near<R>(s, t1, t2, inb, sp, order2, v) ? v : fm_update_octants<R>(s, t1, t2, inb, sp, order2);
 }
 
 // ---------------------------------------------------------------------------
@@ -420,63 +489,10 @@ FM_HD float fm_narrow(double v)
 #endif
 }
 
-// One term of an octant: key, e, spacing and weight, in single precision.
+// One term of an octant in single precision: key, e, weight, one-term solution.
 struct ScreenTerm {
-    float k, e, g, w;
+    float k, e, w, x;
 };
-
-// An octant's (or subset's) screened value: x; whether it stands; whether all
-// three terms enter; its earliest key.
-struct Screened {
-    float x, k0;
-    bool stands, three;
-};
-
-FM_HD void fm_screen_swap(ScreenTerm &a, ScreenTerm &b)
-{
-    const bool p = b.k < a.k;
-    const ScreenTerm t = a;
-    a.k = p ? b.k : a.k; a.e = p ? b.e : a.e; a.g = p ? b.g : a.g; a.w = p ? b.w : a.w;
-    b.k = p ? t.k : b.k; b.e = p ? t.e : b.e; b.g = p ? t.g : b.g; b.w = p ? t.w : b.w;
-}
-
-// a, b, c sorted by key
-FM_HD Screened fm_screen(float s, float s2, const ScreenTerm &a, const ScreenTerm &b, const ScreenTerm &c)
-{
-    Screened r;
-    r.k0 = a.k;
-    const float x0 = fm_fma<float>(s, a.g, a.e);
-    float x = x0;
-    bool three = false;
-    // the second term clearly out, or clearly in whichever of the first two
-    // comes first
-    bool in2 = b.k < x0;
-    bool ok = in2 ? b.k < x0 * (1.0f - kScreen) : b.k > x0 * (1.0f + kScreen);
-    const bool near01 = b.k * (1.0f - kScreen) <= a.k;
-    ok = ok && !(near01 && !(b.k * (1.0f + kScreen) < fm_min(x0, fm_fma<float>(s, b.g, b.e))));
-    if (in2) {
-        const float A = a.w + b.w, B = fm_fma<float>(a.w, a.e, b.w * b.e);
-        const float d01 = a.e - b.e, q01 = a.w * b.w * d01 * d01;
-        const float D = A * s2 - q01;
-        x = Fast<float>::div(B + Fast<float>::sqrt(fm_max(D, 0.0f)), A);
-        ok = ok && D >= A * s2 * (1.0f / 32.0f);
-        three = c.k < x;
-        ok = ok && (three ? c.k < x * (1.0f - kScreen) : c.k > x * (1.0f + kScreen));
-        const bool near12 = c.k * (1.0f - kScreen) <= b.k;
-        ok = ok && !(near12 && (b.e != b.k || c.e != c.k));
-        if (three) {
-            const float A3 = A + c.w, B3 = fm_fma<float>(c.w, c.e, B);
-            const float d02 = a.e - c.e, d12 = b.e - c.e;
-            const float D3 = A3 * s2 - (q01 + c.w * (a.w * d02 * d02 + b.w * d12 * d12));
-            x = Fast<float>::div(B3 + Fast<float>::sqrt(fm_max(D3, 0.0f)), A3);
-            ok = ok && D3 >= A3 * s2 * (1.0f / 32.0f);
-        }
-    }
-    r.x = x;
-    r.stands = ok;                                    // (false for NaN)
-    r.three = three && ok;
-    return r;
-}
 
 // The double-precision causal solve of one octant: terms in axis order, dt
 // the keys, dd = t1 - t2 where the axis is second order (o2), h and w the
@@ -530,64 +546,177 @@ FM_HD double fm_octant(double s, const double dt[3], const double dd[3], unsigne
     return x;
 }
 
+// A pair's screened solve: its value x, whether its second term enters (on)
+// and whether the value stands (ok); Q = w_i w_j (e_i - e_j)^2.
+struct ScreenPair {
+    float x, Q;
+    bool on, ok;
+};
+
+FM_HD ScreenPair fm_screen_pair(float s2, const ScreenTerm &u, const ScreenTerm &v)
+{
+    ScreenPair r;
+    const float A = u.w + v.w, B = fm_fma<float>(u.w, u.e, v.w * v.e), d = u.e - v.e;
+    r.Q = u.w * v.w * d * d;
+    const float D = fm_fma<float>(A, s2, -r.Q);
+    const float x = Fast<float>::div(B + Fast<float>::sqrt(fm_max(D, 0.0f)), A);
+    const float xf = v.k < u.k ? v.x : u.x, kl = fm_max(u.k, v.k), kf = fm_min(u.k, v.k);
+    r.on = kl < xf;
+    const bool clear = r.on ? kl < xf * (1.0f - kScreen) && D >= A * s2 * (1.0f / 32.0f) : kl > xf * (1.0f + kScreen);
+    // (keys that the sort could exchange: the second has to enter either way)
+    const bool tie = kl * (1.0f - kScreen) <= kf && !(kl * (1.0f + kScreen) < fm_min(u.x, v.x));
+    r.ok = clear && !tie;
+    r.x = r.on ? x : xf;
+    return r;
+}
+
+// A triple's, from its pairs: x, whether it stands, whether all three terms
+// enter.  (Which pair comes first matters for the decisions only; sums and
+// discriminant are the same in any order.)
+FM_HD bool fm_screen_triple(float s2, const ScreenTerm &a, const ScreenTerm &b, const ScreenTerm &c, const ScreenPair &ab,
+                            const ScreenPair &ac, const ScreenPair &bc, float &x, bool &three)
+{
+    const float bcmax = fm_max(b.k, c.k);
+    const bool al = bcmax < a.k, cb = c.k < b.k;             // a last; c before b
+    const float kL = fm_max(a.k, bcmax), kM = al ? bcmax : fm_max(a.k, fm_min(b.k, c.k));
+    const float x2 = al ? bc.x : (cb ? ac.x : ab.x);
+    const bool on2 = al ? bc.on : (cb ? ac.on : ab.on);
+    bool ok = al ? bc.ok : (cb ? ac.ok : ab.ok);
+    const float A = a.w + b.w + c.w, B = fm_fma<float>(a.w, a.e, fm_fma<float>(b.w, b.e, c.w * c.e));
+    const float D = fm_fma<float>(A, s2, -(ab.Q + ac.Q + bc.Q));
+    const float x3 = Fast<float>::div(B + Fast<float>::sqrt(fm_max(D, 0.0f)), A);
+    const bool on3 = on2 && kL < x2;
+    if (on2)
+        ok = ok && (on3 ? kL < x2 * (1.0f - kScreen) && D >= A * s2 * (1.0f / 32.0f) : kL > x2 * (1.0f + kScreen)) &&
+             !(kL * (1.0f - kScreen) <= kM);
+    x = on3 ? x3 : x2;
+    three = on3 && ok;
+    return ok;
+}
+
+// The seven subsets of three terms, screened (bits: 0 D, 1 X, 2 Z, 3 DX, 4 DZ,
+// 5 XZ, 6 DXZ): those that can be the least among the ones in `in`; three:
+// DXZ's three terms clearly enter.
+FM_HD unsigned fm_screen7(float s, const ScreenTerm t[3], unsigned in, bool &three)
+{
+    const float INF = Lim<float>::inf();
+    const float s2 = s * s;
+    const ScreenPair p[3] = {fm_screen_pair(s2, t[0], t[1]), fm_screen_pair(s2, t[0], t[2]),
+                             fm_screen_pair(s2, t[1], t[2])};
+    float xt;
+    const bool ok = fm_screen_triple(s2, t[0], t[1], t[2], p[0], p[1], p[2], xt, three);
+    const float k0 = fm_min(fm_min(t[0].k, t[1].k), t[2].k);
+    const float lo[7] = {t[0].x, t[1].x, t[2].x, p[0].ok ? p[0].x : fm_min(t[0].k, t[1].k),
+                         p[1].ok ? p[1].x : fm_min(t[0].k, t[2].k), p[2].ok ? p[2].x : fm_min(t[1].k, t[2].k), ok ? xt : k0};
+    const bool stands[7] = {true, true, true, p[0].ok, p[1].ok, p[2].ok, ok};
+    float m = INF;
+#pragma unroll
+    for (int j = 0; j < 7; ++j) m = ((in >> j) & 1u) && stands[j] ? fm_min(m, lo[j]) : m;
+    const float cut = m * (1.0f + 2.0f * kScreen);
+    unsigned need = 0;
+#pragma unroll
+    for (int j = 0; j < 7; ++j) need |= lo[j] <= cut && lo[j] < INF ? 1u << j : 0u;
+    return need & in;
+}
+
+// The least of the subsets in `need`, solved in double precision.
+FM_HD double fm_solve7(double s, const double dt[3], const double dd[3], unsigned o2, const Spacing<double> &sp,
+                       unsigned need, bool three)
+{
+    const double INF = Lim<double>::inf();
+    double best = INF;
+    while (need) {
+        const unsigned bit = need & (0u - need);
+        need ^= bit;
+        // D in 0, 3, 4, 6; X in 1, 3, 5, 6; Z in 2, 4, 5, 6
+        const double kt[3] = {(bit & 0x59u) ? dt[0] : INF, (bit & 0x6au) ? dt[1] : INF, (bit & 0x74u) ? dt[2] : INF};
+        const double v = fm_octant(s, kt, dd, o2, sp, bit == 0x40u && three);
+        best = fm_less(v, best) ? v : best;
+    }
+    return best;
+}
+
+// Which subsets' octants lie inside the grid: each takes the near side on its
+// axes and the far side on the others (n, f: bit a of each).
+FM_HD unsigned fm_inside7(unsigned n, unsigned f)
+{
+    unsigned in = 0;
+    const unsigned sets[7] = {1u, 2u, 4u, 3u, 5u, 6u, 7u};
+#pragma unroll
+    for (int j = 0; j < 7; ++j) in |= (((n & sets[j]) | (f & ~sets[j])) & 7u) == 7u ? 1u << j : 0u;
+    return in;
+}
+
+// One side's term: keys and differences in double, the screen's in single.
+FM_HD void fm_side(float s, double t1, double t2, double tmin, double h, double w, int order2, double &dt, double &dd,
+                   bool &o2, ScreenTerm &t)
+{
+    o2 = order2 && fm_less(t2, t1);
+    dt = t1 - tmin;
+    dd = o2 ? t1 - t2 : 0.0;
+    const float hf = fm_narrow(h), wf = fm_narrow(w);
+    t.k = fm_narrow(dt);
+    t.e = o2 ? fm_fma<float>(fm_narrow(dd), 1.0f / 3.0f, t.k) : t.k;
+    t.w = o2 ? wf * 2.25f : wf;
+    t.x = fm_fma<float>(s, o2 ? hf * (2.0f / 3.0f) : hf, t.e);
+}
+
+// fm_update in double precision: all eight octants screened, in straight-line
+// code that shares the twelve pairs (an octant's value is its triple's), then
+// those that can be the least solved in double.  (The short form with a
+// fallback loses here: along a near tie's axis a warp seldom has all lanes
+// in it, and both forms run -- rounds and extra sweeps of the two-event
+// 192x224x224 solve 192 and 93 ms against 157 and 57.)
 template <>
 FM_HD double fm_update<double>(double s, const double t1[6], const double t2[6], unsigned inb,
                                const Spacing<double> &sp, int order2)
 {
     const double INF = Lim<double>::inf();
+    const float INFF = Lim<float>::inf();
     double tmin = INF;
 #pragma unroll
     for (int d = 0; d < 6; ++d) tmin = fm_less(t1[d], tmin) ? t1[d] : tmin;
     if (!fm_less(tmin, INF)) return INF;
-    float hf[3], wf[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        hf[a] = fm_narrow(sp.h[a]);
-        wf[a] = fm_narrow(sp.w[a]);
-    }
-    const float sf = fm_narrow(s), s2f = sf * sf;
+    const float sf = fm_narrow(s), s2 = sf * sf;
     double dt[6], dd[6];
     unsigned o2 = 0;
     ScreenTerm t[6];
 #pragma unroll
     for (int d = 0; d < 6; ++d) {
-        const int a = d >> 1;
-        const bool o = order2 && fm_less(t2[d], t1[d]);
-        dt[d] = t1[d] - tmin;
-        dd[d] = o ? t1[d] - t2[d] : 0.0;
+        bool o;
+        fm_side(sf, t1[d], t2[d], tmin, sp.h[d >> 1], sp.w[d >> 1], order2, dt[d], dd[d], o, t[d]);
         o2 |= o ? 1u << d : 0u;
-        t[d].k = fm_narrow(dt[d]);
-        t[d].e = o ? fm_fma<float>(fm_narrow(dd[d]), 1.0f / 3.0f, t[d].k) : t[d].k;
-        t[d].g = o ? hf[a] * (2.0f / 3.0f) : hf[a];
-        t[d].w = o ? wf[a] * 2.25f : wf[a];
     }
-    // octant q: bit 0 the radial side, bit 1 theta, bit 2 phi
-    float lo[8];           // least value the octant can have, as far as the screen tells
+    // pairs of sides: radial with theta, radial with phi, theta with phi
+    ScreenPair rx[4], rz[4], xz[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        rx[q] = fm_screen_pair(s2, t[q & 1], t[2 + (q >> 1)]);
+        rz[q] = fm_screen_pair(s2, t[q & 1], t[4 + (q >> 1)]);
+        xz[q] = fm_screen_pair(s2, t[2 + (q & 1)], t[4 + (q >> 1)]);
+    }
+    // octant q: bit 0 the radial side, bit 1 theta, bit 2 phi; the least value
+    // each can have, as far as the screen tells
+    float lo[8], m = INFF;
     unsigned three = 0;
-    float m = Lim<float>::inf();
 #pragma unroll
-    for (int lat = 0; lat < 4; ++lat) {
-        ScreenTerm a = t[2 + (lat & 1)], b = t[4 + (lat >> 1)];
-        fm_screen_swap(a, b);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int q = r | (lat << 1);
-            const unsigned om = (1u << r) | (4u << (lat & 1)) | (16u << (lat >> 1));
-            ScreenTerm x = t[r], y = a, z = b;
-            fm_screen_swap(x, y);
-            fm_screen_swap(y, z);
-            const Screened v = fm_screen(sf, s2f, x, y, z);
-            const bool in = (inb & om) == om;
-            lo[q] = in ? (v.stands ? v.x : v.k0) : Lim<float>::inf();
-            m = in && v.stands ? fm_min(m, v.x) : m;
-            three |= v.three ? 1u << q : 0u;
-        }
+    for (int q = 0; q < 8; ++q) {
+        const int r = q & 1, x = (q >> 1) & 1, z = q >> 2;
+        const unsigned om = (1u << r) | (4u << x) | (16u << z);
+        float v;
+        bool th;
+        const bool ok = fm_screen_triple(s2, t[r], t[2 + x], t[4 + z], rx[r | x << 1], rz[r | z << 1], xz[x | z << 1], v, th);
+        const float k0 = fm_min(fm_min(t[r].k, t[2 + x].k), t[4 + z].k);
+        const bool in = (inb & om) == om;
+        lo[q] = in ? (ok ? v : k0) : INFF;
+        m = in && ok ? fm_min(m, v) : m;
+        three |= th ? 1u << q : 0u;
     }
     // (an octant outside the grid, or with no neighbour set, has lo = +inf)
     const float cut = m * (1.0f + 2.0f * kScreen);
     unsigned need = 0;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) need |= lo[q] <= cut && lo[q] < Lim<float>::inf() ? 1u << q : 0u;
+    for (int q = 0; q < 8; ++q) need |= lo[q] <= cut && lo[q] < INFF ? 1u << q : 0u;
     double best = INF;
     while (need) {
         const unsigned bit = need & (0u - need);
@@ -603,75 +732,31 @@ FM_HD double fm_update<double>(double s, const double t1[6], const double t2[6],
     return tmin + best;
 }
 
-// The upstream-only update, screened likewise over its seven subsets (bit 0
-// down, bit 1 theta, bit 2 phi).
 template <>
 FM_HD double fm_update_upstream<double>(double s, double tD, double tD2, double tX, double tX2, double tZ, double tZ2,
                                         bool inD, bool inU, bool inXu, bool inXd, bool inZu, bool inZd,
                                         const Spacing<double> &sp, int order2)
 {
     const double INF = Lim<double>::inf();
-    const float INFF = Lim<float>::inf();
     double tmin = fm_less(tX, tD) ? tX : tD;
     tmin = fm_less(tZ, tmin) ? tZ : tmin;
     if (!fm_less(tmin, INF)) return INF;
     const double t1[3] = {tD, tX, tZ}, t2[3] = {tD2, tX2, tZ2};
-    const float sf = fm_narrow(s), s2f = sf * sf;
+    const float sf = fm_narrow(s);
     double dt[3], dd[3];
     unsigned o2 = 0;
     ScreenTerm t[3];
-    float x1[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const bool o = order2 && fm_less(t2[a], t1[a]);
-        dt[a] = t1[a] - tmin;
-        dd[a] = o ? t1[a] - t2[a] : 0.0;
+        bool o;
+        fm_side(sf, t1[a], t2[a], tmin, sp.h[a], sp.w[a], order2, dt[a], dd[a], o, t[a]);
         o2 |= o ? 1u << a : 0u;
-        const float h = fm_narrow(sp.h[a]), w = fm_narrow(sp.w[a]);
-        t[a].k = fm_narrow(dt[a]);
-        t[a].e = o ? fm_fma<float>(fm_narrow(dd[a]), 1.0f / 3.0f, t[a].k) : t[a].k;
-        t[a].g = o ? h * (2.0f / 3.0f) : h;
-        t[a].w = o ? w * 2.25f : w;
-        x1[a] = fm_fma<float>(sf, t[a].g, t[a].e);
     }
-    float lo[7];
-    unsigned three = 0;
-    float m = INFF;
-    // singles stand as they are
-    const bool c1[3] = {inD && inXd && inZd, inU && inXu && inZd, inU && inXd && inZu};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        lo[a] = c1[a] ? x1[a] : INFF;
-        m = fm_min(m, lo[a]);
-    }
-    const ScreenTerm none = {INFF, INFF, 1.0f, 1.0f};
-    const bool c2[4] = {inD && inXu && inZd, inD && inXd && inZu, inU && inXu && inZu, inD && inXu && inZu};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        // DX, DZ, XZ, DXZ
-        ScreenTerm x = t[j == 2 ? 1 : 0], y = t[j == 0 || j == 3 ? 1 : 2], z = j == 3 ? t[2] : none;
-        if (j == 3) fm_screen_swap(y, z);
-        fm_screen_swap(x, y);
-        if (j == 3) fm_screen_swap(y, z);
-        const Screened v = fm_screen(sf, s2f, x, y, z);
-        lo[3 + j] = c2[j] ? (v.stands ? v.x : v.k0) : INFF;
-        m = c2[j] && v.stands ? fm_min(m, v.x) : m;
-        if (j == 3 && v.three) three = 1;
-    }
-    const float cut = m * (1.0f + 2.0f * kScreen);
-    unsigned need = 0;
-#pragma unroll
-    for (int j = 0; j < 7; ++j) need |= lo[j] <= cut && lo[j] < INFF ? 1u << j : 0u;
-    double best = INF;
-    while (need) {
-        const unsigned bit = need & (0u - need);
-        need ^= bit;
-        // D in 0, 3, 4, 6; X in 1, 3, 5, 6; Z in 2, 4, 5, 6
-        const double kt[3] = {(bit & 0x59u) ? dt[0] : INF, (bit & 0x6au) ? dt[1] : INF, (bit & 0x74u) ? dt[2] : INF};
-        const double v = fm_octant(s, kt, dd, o2, sp, bit == 0x40u && three);
-        best = fm_less(v, best) ? v : best;
-    }
-    return tmin + best;
+    bool three;
+    const unsigned n = (inD ? 1u : 0u) | (inXu ? 2u : 0u) | (inZu ? 4u : 0u);
+    const unsigned f = (inU ? 1u : 0u) | (inXd ? 2u : 0u) | (inZd ? 4u : 0u);
+    const unsigned need = fm_screen7(sf, t, fm_inside7(n, f), three);
+    return tmin + fm_solve7(s, dt, dd, o2, sp, need, three);
 }
 
 }  // namespace fm3dt
