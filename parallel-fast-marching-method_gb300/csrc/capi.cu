@@ -184,79 +184,28 @@ int ensure_planes(fm3dt_ctx *ctx, int shape)
     return FM3DT_OK;
 }
 
-// Hyperplanes s' + x' + z' = h of a streaming sweep's work items: height
-// segment s' (counted upward), column blocks x', z' in swept coordinates,
-// packed s'<<24 | x'<<12 | z'.
-int ensure_block_planes(fm3dt_ctx *ctx, int sweep_shape, int nseg, const fm3dt_ctx::Planes **out)
+// Hyperplanes x' + z' = h of a streaming sweep's column blocks in swept
+// coordinates, packed x'<<12 | z'.
+int ensure_block_planes(fm3dt_ctx *ctx, int sweep_shape, const fm3dt_ctx::Planes **out)
 {
     for (const auto &P : ctx->block_planes)
-        if (P.shape == sweep_shape && P.nseg == nseg) {
+        if (P.shape == sweep_shape) {
             *out = &P;
             return FM3DT_OK;
         }
     const StreamShape ss = kStreamShapes[sweep_shape - kNumShapes];
     const int nbx = (ctx->g.nnx + ss.sx - 1) / ss.sx, nbz = (ctx->g.nnz + ss.sz - 1) / ss.sz;
-    if (nbx > 4095 || nbz > 4095 || nseg > 127) return fail(ctx, FM3DT_EINVAL, "too many column blocks or segments");
+    if (nbx > 4095 || nbz > 4095) return fail(ctx, FM3DT_EINVAL, "too many column blocks");
     fm3dt_ctx::Planes P;
     P.shape = sweep_shape;
-    P.nseg = nseg;
-    const int H = nseg + nbx + nbz - 2;
     std::vector<int> flat;
-    P.off.assign(H, 0);
-    P.cnt.assign(H, 0);
-    for (int h = 0; h < H; ++h) {
-        P.off[h] = (int)flat.size();
-        for (int s = 0; s < nseg && s <= h; ++s)
-            for (int b = std::max(0, h - s - nbz + 1); b <= std::min(h - s, nbx - 1); ++b)
-                flat.push_back((s << 24) | (b << 12) | (h - s - b));
-        P.cnt[h] = (int)flat.size() - P.off[h];
-    }
+    for (int h = 0; h < nbx + nbz - 1; ++h)
+        for (int b = std::max(0, h - nbz + 1); b <= std::min(h, nbx - 1); ++b) flat.push_back((b << 12) | (h - b));
     CK(cudaMalloc(&P.d_tiles, flat.size() * sizeof(int)));
     CK(cudaMemcpy(P.d_tiles, flat.data(), flat.size() * sizeof(int), cudaMemcpyHostToDevice));
     ctx->block_planes.push_back(std::move(P));
     *out = &ctx->block_planes.back();
     return FM3DT_OK;
-}
-
-// Height segments for a streaming sweep over nitems events: enough work
-// items per launch to fill the GPU once, each segment at least 16 layers.
-// Height segments for a streaming sweep of nitems events: the count that
-// minimises a model of its time.  Hyperplane h of the items (segment s,
-// column block (x', z')) with s + x' + z' = h is one launch; its items run in
-// ceil(items / sgrid) waves of seg_len + SX + SZ - 2 steps each (the
-// wavefront ramp), plus a few steps' worth of launch gap.  More segments give
-// a launch more items (fewer idle SMs) but more launches and more ramp.
-int stream_segments(const fm3dt_ctx *ctx, int nitems, int nbx, int nbz, int sgrid, int ramp)
-{
-    const int nnr = ctx->g.nnr;
-    constexpr double kLaunchSteps = 4.0;
-    // an item fills its ring (five layers and the first prefetch) before its
-    // first step: about six steps' worth of loads
-    constexpr int kFillSteps = 6;
-    // blocks per lateral hyperplane (x' + z' = d)
-    std::vector<long long> lat(nbx + nbz - 1, 0);
-    for (int d = 0; d < nbx + nbz - 1; ++d)
-        lat[d] = std::min(d, nbx - 1) - std::max(0, d - (nbz - 1)) + 1;
-    int best = 1;
-    double best_t = 0.0;
-    for (int nseg = 1; nseg <= std::max(1, nnr / 8); nseg *= 2) {
-        const int seg_len = (nnr + nseg - 1) / nseg;
-        double t = 0.0;
-        for (int h = 0; h < nbx + nbz - 1 + nseg - 1; ++h) {
-            long long cnt = 0;
-            for (int sg = 0; sg < nseg; ++sg) {
-                const int d = h - sg;
-                if (d >= 0 && d < nbx + nbz - 1) cnt += lat[d];
-            }
-            const long long items = cnt * (long long)nitems;
-            t += (double)((items + sgrid - 1) / sgrid) * (seg_len + ramp + kFillSteps) + kLaunchSteps;
-        }
-        if (nseg == 1 || t < best_t) {
-            best = nseg;
-            best_t = t;
-        }
-    }
-    return best;
 }
 
 // The field as a 4-D tensor (phi, theta, r, event) for TMA copies of a round
@@ -333,25 +282,6 @@ const CUtensorMap *field_tensor_map(fm3dt_ctx *ctx, int shape)
 #ifndef FM_TIE_SKIP
 #define FM_TIE_SKIP 1
 #endif
-//   FM_SWEEP_FLOW          a tracked extra sweep as one launch whose items start
-//                          when their upstream neighbours are done (instead of
-//                          one launch per hyperplane)
-#ifndef FM_SWEEP_FLOW
-#define FM_SWEEP_FLOW 1
-#endif
-//   FM_FLOW_FIRST          ... the first tracked sweep of a chain too
-#ifndef FM_FLOW_FIRST
-#define FM_FLOW_FIRST 1
-#endif
-//   FM_FLOW_SHARE_FIRST    percent of the resident slots a one-launch pass on stream2
-//   FM_FLOW_SHARE          takes: the chain's first tracked sweep (beside the other part's
-//                          certification), the later ones
-#ifndef FM_FLOW_SHARE_FIRST
-#define FM_FLOW_SHARE_FIRST 75
-#endif
-#ifndef FM_FLOW_SHARE
-#define FM_FLOW_SHARE 75
-#endif
 #ifndef FM_ROUND0_PER_TILE
 #define FM_ROUND0_PER_TILE 1
 #endif
@@ -368,9 +298,6 @@ const CUtensorMap *field_tensor_map(fm3dt_ctx *ctx, int shape)
 #define FM_OVERLAP_MAIN 1
 #endif
 
-#ifndef FM_SWEEP_GRAPHS
-#define FM_SWEEP_GRAPHS 1
-#endif
 
 // How a solve starts: from boundary frames (initialisation, sweep, rounds),
 // from the current fields (resume: rounds with every tile active), or from
@@ -468,39 +395,35 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     const int sidx = streaming ? ctx->sweep_shape - kNumShapes : 0;
     const int nbx = (g.nnx + kStreamShapes[sidx].sx - 1) / kStreamShapes[sidx].sx;
     const int nbz = (g.nnz + kStreamShapes[sidx].sz - 1) / kStreamShapes[sidx].sz;
-    // resident one-warp CTAs of the streaming sweep
-    auto stream_grid = [&](bool flow) {
-        return streaming ? std::max(1, ctx->prec == FM3DT_FP64 ? occupancy_stream_f64(sidx, flow)
-                                                               : occupancy_stream_f32(sidx, flow)) * sm_count()
-                         : 1;
+    // Events swept side by side (a group): as many as fill the resident warps
+    // one and a half times with two hyperplanes of blocks.  A block holds its
+    // warp while it waits for the blocks upstream; with fewer events, more
+    // hyperplanes of each are under way, whose warps mostly wait (near-tie
+    // sweeps of 89 events on 192x224x224, 17 at a time: 50 ms instead of 23);
+    // with more, the halo columns have left L2 when they are read.
+    auto sweep_group = [&](int nitems, double slots) {
+        const double plane = (double)nbx * nbz / (nbx + nbz - 1);
+        return (int)std::min<double>(nitems, std::ceil(0.75 * slots / plane));
     };
-    // The main sweep of nitems events (events == null: all), one launch.  The
-    // events of a group are swept side by side: as many as fill the resident
-    // warps one and a half times with the blocks that can be under way at
-    // once (a block trails those upstream by ~14 steps, so an event has
-    // nnr / 14 hyperplanes of blocks under way), no more, so that the halo
-    // columns are still in L2 when the next hyperplane reads them.
+    // The main sweep of nitems events (events == null: all)
     auto front_pass = [&](int nitems, const int *events, cudaStream_t st) -> int {
         sweep_nodes += (int64_t)nitems * (int64_t)ctx->N;
         const fm3dt_ctx::Planes *P = nullptr;
-        const int rc = ensure_block_planes(ctx, ctx->sweep_shape, 1, &P);
+        const int rc = ensure_block_planes(ctx, ctx->sweep_shape, &P);
         if (rc) return rc;
         const int occ = ctx->prec == FM3DT_FP64 ? occupancy_front_f64(sidx) : occupancy_front_f32(sidx);
         const double slots = (double)std::max(1, occ) * sm_count();
-        const int nblocks = nbx * nbz, planes = nbx + nbz - 1;
-        const double under_way = (double)nblocks / planes * std::min(planes, g.nnr / 14 + 1);
-        const int group = (int)std::min<double>(nitems, std::ceil(1.5 * slots / under_way));
         const int si = st == ctx->stream2 ? 1 : 0;
         CK(cudaMemsetAsync(ctx->d_next + si, 0, sizeof(unsigned), st));
         auto fill = [&](auto &a) {
             a.blocks = P->d_tiles;
-            a.nblocks = nblocks;
+            a.nblocks = nbx * nbz;
             a.dir = ctx->d_dir;
             a.events = events;
             a.nev = nitems;
-            a.group = group;
+            a.group = sweep_group(nitems, slots);
             a.nbx = nbx; a.nbz = nbz;
-            a.count = (unsigned)nblocks * (unsigned)nitems;
+            a.count = (unsigned)(nbx * nbz) * (unsigned)nitems;
             a.next = ctx->d_next + si;
             // (all blocks resident at once: bound by the critical path, see
             // front.cuh for both sides measured)
@@ -523,159 +446,100 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         ctx->launches += 1;
         return FM3DT_OK;
     };
-    // One streaming sweep of nitems events (events == null: all), lateral
+    // chunks of at least 4 layers, at most 32 of them
+    int act_shift = 2;
+    while (((g.nnr - 1) >> act_shift) >= 32) ++act_shift;
+    // Certification of the events swept exactly once: the first round of those
+    // that get no extra sweeps recomputes only the nodes it marks, on the tiles
+    // it appends to list 0; the first extra sweep of the near-tie events runs
+    // only where it marks nodes (act: their chunk masks)
+    auto certify = [&](const int *events, int n, cudaStream_t st, unsigned *act = nullptr) {
+        auto fill = [&](auto &ca, const auto &f) {
+            ca.f = f;
+            ca.events = events; ca.nev = n;
+            ca.dir = ctx->d_dir;
+            ca.cert = ctx->d_cert; ca.cert_nw = ctx->cert_nw;
+            ca.tr = ts.tr; ca.tx = ts.tx; ca.tz = ts.tz;
+            ca.flag = ctx->d_flag; ca.list = ctx->d_list[0]; ca.count = ctx->d_count[0];
+            ca.act = act;
+            ca.act_shift = act_shift;
+            ca.bsx = kStreamShapes[sidx].sx; ca.bsz = kStreamShapes[sidx].sz;
+            ca.nbx = nbx; ca.nbz = nbz;
+        };
+        if (ctx->prec == FM3DT_FP64) {
+            CertifyArgs<double> ca{};
+            fill(ca, f64);
+            launch_certify_f64(ca, st);
+        } else {
+            CertifyArgs<float> ca{};
+            fill(ca, f32);
+            launch_certify_f32(ca, st);
+        }
+        ctx->launches += 1;
+    };
+    // One more sweep of nitems events (events == null: all), lateral
     // directions flipped by `flip`; with `flag`, changed nodes queue their
-    // tiles (and face neighbours) on list/count for the rounds.
-    // `recurs`: a pass that recurs from solve to solve (kept as a graph).
-    // `act`: the item activity of a chain of sweeps (this sweep's, the
-    // previous one's or null), see StreamArgs.
-    auto stream_pass = [&](int nitems, const int *events, int flip, int nseg, int *flag, int *list,
-                           int *count, cudaStream_t st, bool recurs,
+    // tiles (and face neighbours) on list/count for the rounds.  `act`: the
+    // activity of a chain of sweeps (this sweep's, the previous one's or
+    // null), see StreamArgs.
+    auto stream_pass = [&](int nitems, const int *events, int flip, int *flag, int *list, int *count, cudaStream_t st,
                            unsigned *act_cur = nullptr, const unsigned *act_prev = nullptr,
                            unsigned long long *act_items = nullptr) -> int {
         sweep_nodes += (int64_t)nitems * (int64_t)ctx->N;
-        const int sgrid = stream_grid(false);
-        if (nseg <= 0) nseg = stream_segments(ctx, nitems, nbx, nbz, sgrid, kStreamShapes[sidx].sx + kStreamShapes[sidx].sz - 2);
-        nseg = std::min(nseg, g.nnr);
-        // (no empty segment: 130 layers in 16 segments of 9 fill only 15; an
-        // item above the grid would read parameters outside their arrays)
-        const int seg_len = (g.nnr + nseg - 1) / nseg;
-        nseg = (g.nnr + seg_len - 1) / seg_len;
-        const fm3dt_ctx::Planes *PP = nullptr;
-        int rc = ensure_block_planes(ctx, ctx->sweep_shape, nseg, &PP);
+        const fm3dt_ctx::Planes *P = nullptr;
+        const int rc = ensure_block_planes(ctx, ctx->sweep_shape, &P);
         if (rc) return rc;
-        const auto &P = *PP;
-        // (items of one layer or column would miss a 2-deep neighbour)
-        const bool track = act_cur && seg_len >= 2 && kStreamShapes[sidx].sx >= 2;
-        // One launch for the whole pass (FM_SWEEP_FLOW): items start as their
-        // upstream neighbours finish, with a done flag per item and a queue
-        // counter of the pass's stream, both zeroed ahead of the launch.  For
-        // the tracked sweeps after a chain's first, whose few active items
-        // would leave most of each hyperplane's launch idle; passes that run
-        // every item keep one launch per hyperplane, which shares the GPU with
-        // the other stream's work (a one-launch pass holds every SM slot).
         const int si = st == ctx->stream2 ? 1 : 0;
-        const bool flow = FM_SWEEP_FLOW && streaming && track && (act_prev != nullptr || FM_FLOW_FIRST);
-        const int nblocks = P.off.empty() ? 0 : P.off.back() + P.cnt.back();
-        const size_t done_n = (size_t)nitems * (size_t)((g.nnr + seg_len - 1) / seg_len) * (size_t)nbx * (size_t)nbz;
-        if (flow && done_n * sizeof(unsigned) > ctx->done_bytes[si]) {
+        const size_t words = (size_t)nitems * (size_t)nbx * (size_t)nbz;
+        if (words * sizeof(unsigned long long) > ctx->prog_bytes[si]) {
             CK(cudaStreamSynchronize(st));
-            cudaFree(ctx->d_done[si]);
-            ctx->d_done[si] = nullptr;
-            ctx->done_bytes[si] = 0;
-            CK(cudaMalloc(&ctx->d_done[si], done_n * sizeof(unsigned)));
-            ctx->done_bytes[si] = done_n * sizeof(unsigned);
+            cudaFree(ctx->d_prog[si]);
+            ctx->d_prog[si] = nullptr;
+            ctx->prog_bytes[si] = 0;
+            CK(cudaMalloc(&ctx->d_prog[si], words * sizeof(unsigned long long)));
+            ctx->prog_bytes[si] = words * sizeof(unsigned long long);
         }
-        // (on stream2, beside the other part's work, a share of the resident
-        // slots: a one-launch pass holds its slots to the end)
-        const int fgrid = flow ? (int)std::min<long long>((long long)nblocks * nitems,
-                                                          std::max(1, stream_grid(true) *
-                                                                          (si ? (act_prev ? FM_FLOW_SHARE
-                                                                                          : FM_FLOW_SHARE_FIRST)
-                                                              : 100) / 100))
-                               : 0;
-        // the pass's launches: one (flow), else one per hyperplane (two with a
-        // tracked previous sweep)
-        const int nlaunch = flow ? 1 : (int)P.off.size() * (track && act_prev ? 2 : 1);
-        // (returns the first error of the flags' and counter's zeroing; the
-        // launches' errors surface at the next check)
-        auto enqueue = [&]() -> cudaError_t {
-            cudaError_t ez = cudaSuccess;
-            if (flow) {
-                ez = cudaMemsetAsync(ctx->d_done[si], 0, done_n * sizeof(unsigned), st);
-                if (ez == cudaSuccess) ez = cudaMemsetAsync(ctx->d_next + si, 0, sizeof(unsigned), st);
-                if (ez != cudaSuccess) return ez;
-            }
-            for (size_t h = 0; h < (flow ? (size_t)1 : P.off.size()); ++h) {
-                const long long items = (long long)P.cnt[h] * nitems;
-                const int grid = flow ? fgrid : (int)std::min<long long>(items, sgrid);
-                auto fill = [&](auto &a) {
-                    a.hp_blocks = P.d_tiles; a.hoff = flow ? 0 : P.off[h]; a.hcount = flow ? nblocks : P.cnt[h];
-                    a.flow = flow ? 1 : 0;
-                    a.done = flow ? ctx->d_done[si] : nullptr;
-                    a.done_n = flow ? done_n : 0;
-                    a.next = flow ? ctx->d_next + si : nullptr;
-                    a.dir = ctx->d_dir; a.nev = nitems; a.nbx = nbx; a.nbz = nbz;
-                    a.events = events;
-                    a.flip = flip;
-                    a.seg_len = seg_len;
-                    a.flag = flag;
-                    a.list = list; a.count = count;
-                    a.tr = ts.tr; a.tx = ts.tx; a.tz = ts.tz;
-                    a.ntr = ntr; a.ntx = ntx; a.ntz = ntz; a.tiles_per_event = tpe;
-                    a.act_cur = track ? act_cur : nullptr;
-                    a.act_prev = track ? act_prev : nullptr;
-                    a.act_run = track && !flow ? ctx->d_act[2] : nullptr;
-                    // chunks of at least 4 layers, at most 32 of them per item
-                    a.act_shift = 2;
-                    while (((seg_len - 1) >> a.act_shift) >= 32) ++a.act_shift;
-                    a.act_items = track ? act_items : nullptr;
-                    a.act_n = ctx->act_bytes / sizeof(unsigned);
-                    a.err = ctx->d_err;
-                };
-                if (ctx->prec == FM3DT_FP64) {
-                    StreamArgs<double> a{};
-                    a.f = f64;
-                    fill(a);
-                    launch_stream_f64(sidx, grid, a, st);
-                } else {
-                    StreamArgs<float> a{};
-                    a.f = f32;
-                    fill(a);
-                    launch_stream_f32(sidx, grid, a, st);
-                }
-            }
-            return cudaSuccess;
+        const int occ = ctx->prec == FM3DT_FP64 ? occupancy_stream_f64(sidx) : occupancy_stream_f32(sidx);
+        const int slots = std::max(1, occ) * sm_count();
+        const int grid = (int)std::min<size_t>(words, (size_t)slots);
+        CK(cudaMemsetAsync(ctx->d_prog[si], 0, words * sizeof(unsigned long long), st));
+        CK(cudaMemsetAsync(ctx->d_next + si, 0, sizeof(unsigned), st));
+        auto fill = [&](auto &a) {
+            a.blocks = P->d_tiles;
+            a.nblocks = nbx * nbz;
+            a.dir = ctx->d_dir;
+            a.events = events;
+            a.nev = nitems;
+            a.group = sweep_group(nitems, slots);
+            a.flip = flip;
+            a.nbx = nbx; a.nbz = nbz;
+            a.count = (unsigned)words;
+            a.next = ctx->d_next + si;
+            a.prog = ctx->d_prog[si];
+            a.flag = flag;
+            a.list = list; a.count_out = count;
+            a.tr = ts.tr; a.tx = ts.tx; a.tz = ts.tz;
+            a.ntr = ntr; a.ntx = ntx; a.ntz = ntz; a.tiles_per_event = tpe;
+            a.act_cur = act_cur;
+            a.act_prev = act_prev;
+            a.act_shift = act_shift;
+            a.act_items = act_items;
+            a.err = ctx->d_err;
         };
-        // Passes that recur from solve to solve (the main sweeps and the
-        // near-tie events' extra sweeps; not the re-sweeps, whose event count
-        // varies) run as a graph captured on first use: one launch instead of
-        // one per hyperplane.
-        bool launched = false;
-        if (FM_SWEEP_GRAPHS && recurs && !ctx->sweep_graph_off) {
-            const long long key[fm3dt_ctx::kSweepKey] = {ctx->prec, sidx, nitems, (long long)(intptr_t)events, flip,
-                                                         nseg, (long long)(intptr_t)st, ctx->shape,
-                                                         (long long)(intptr_t)flag, (long long)(intptr_t)list,
-                                                         (long long)(intptr_t)count, (long long)(intptr_t)act_cur,
-                                                         (long long)(intptr_t)act_prev, (long long)(intptr_t)act_items,
-                                                         (long long)(intptr_t)(flow ? ctx->d_done[si] : nullptr)};
-            cudaGraphExec_t exec = nullptr;
-            for (const auto &sg : ctx->sweep_graphs)
-                if (memcmp(sg.key, key, sizeof key) == 0) exec = sg.exec;
-            if (!exec) {
-                cudaGraph_t gr = nullptr;
-                cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-                if (e == cudaSuccess) {
-                    const cudaError_t eq = enqueue();
-                    e = cudaStreamEndCapture(st, &gr);
-                    if (e == cudaSuccess) e = eq;
-                }
-                if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, gr, 0);
-                if (gr) cudaGraphDestroy(gr);
-                if (e != cudaSuccess) {
-                    // launched one by one from now on in this context
-                    (void)cudaGetLastError();
-                    ctx->sweep_graph_off = true;
-                    exec = nullptr;
-                } else {
-                    if (ctx->sweep_graphs.size() >= fm3dt_ctx::kSweepGraphs) {
-                        cudaGraphExecDestroy(ctx->sweep_graphs.front().exec);
-                        ctx->sweep_graphs.erase(ctx->sweep_graphs.begin());
-                    }
-                    fm3dt_ctx::SweepGraph sg;
-                    memcpy(sg.key, key, sizeof key);
-                    sg.exec = exec;
-                    ctx->sweep_graphs.push_back(sg);
-                }
-            }
-            if (exec) {
-                CK(cudaGraphLaunch(exec, st));
-                launched = true;
-            }
+        if (ctx->prec == FM3DT_FP64) {
+            StreamArgs<double> a{};
+            a.f = f64;
+            fill(a);
+            launch_stream_f64(sidx, grid, a, st);
+        } else {
+            StreamArgs<float> a{};
+            a.f = f32;
+            fill(a);
+            launch_stream_f32(sidx, grid, a, st);
         }
-        if (!launched) CK(enqueue());
-        sweep_launches += nlaunch;
-        ctx->launches += nlaunch;
+        CKL();
+        sweep_launches += 1;
+        ctx->launches += 1;
         return FM3DT_OK;
     };
     CK(cudaEventRecord(sw0, s));
@@ -685,8 +549,16 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     bool tie_act = false;              // ties' extra sweeps skip items where nothing changed
     // the activity buffers of extra sweep k: this sweep's and the previous one's
     auto act_cur = [&](int k) { return tie_act ? ctx->d_act[k & 1] : nullptr; };
-    auto act_prev = [&](int k) -> const unsigned * { return tie_act && k > 0 ? ctx->d_act[(k - 1) & 1] : nullptr; };
-    auto act_items = [&](int k) { return tie_act && k < fm3dt_ctx::kMaxTieSweeps ? ctx->d_act_items + 2 * k : nullptr; };
+    // (before the first one: the chunks the certification marks)
+    auto act_prev = [&](int k) -> const unsigned * { return tie_act ? ctx->d_act[(k + 1) & 1] : nullptr; };
+    auto act_start = [&](cudaStream_t st) -> int {
+        if (!tie_act) return FM3DT_OK;
+        CK(cudaMemsetAsync(ctx->d_act[1], 0, ties.size() * (size_t)nbx * (size_t)nbz * sizeof(unsigned), st));
+        certify(ctx->d_events, (int)ties.size(), st, ctx->d_act[1]);
+        CKL();
+        return FM3DT_OK;
+    };
+    auto act_items = [&](int k) { return tie_act && k > 0 && k < fm3dt_ctx::kMaxTieSweeps ? ctx->d_act_items + 2 * k : nullptr; };
     ctx->act_sweeps = 0;
     ctx->tie_sweep_n = 0;
     if (do_sweep && streaming) {
@@ -727,11 +599,10 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
             CK(cudaMemsetAsync(ctx->d_flag, 0, (size_t)nev * tpe * sizeof(int), s));
             CK(cudaMemsetAsync(ctx->d_count[0], 0, sizeof(int), s));
         }
-        // item activity of the near-tie events' extra sweeps: one mask per
-        // (event, segment, column block), for at most 127 segments
-        if (FM_TIE_SKIP && !ties.empty() && ctx->tie_sweeps > 1) {
-            const size_t need = ties.size() * (size_t)std::min(127, g.nnr) * (size_t)nbx * (size_t)nbz *
-                                sizeof(unsigned);
+        // activity of the near-tie events' extra sweeps: one mask per (event,
+        // column block)
+        if (FM_TIE_SKIP && !ties.empty() && ctx->tie_sweeps > 0) {
+            const size_t need = ties.size() * (size_t)nbx * (size_t)nbz * sizeof(unsigned);
             if (need > ctx->act_bytes) {
                 CK(cudaStreamSynchronize(ctx->stream2));
                 for (auto &p : ctx->d_act) {
@@ -768,11 +639,14 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
                 (pass == 2 && !ctx->verify))
                 continue;
             const int nitems = pass == 1 ? (int)ties.size() : nev;
+            if (pass == 1 && pl.k == 0) {
+                const int ra = act_start(s);
+                if (ra) return ra;
+            }
             const int rc = pass == 0 ? front_pass(nev, nullptr, s)
                                      : stream_pass(nitems, pass == 1 ? ctx->d_events : nullptr, pl.flip,
-                                                   pass == 1 ? ctx->tie_segments : ctx->sweep_segments,
                                                    pl.queue ? ctx->d_flag : nullptr, ctx->d_list[0], ctx->d_count[0], s,
-                                                   pass != 2, pass == 1 ? act_cur(pl.k) : nullptr,
+                                                   pass == 1 ? act_cur(pl.k) : nullptr,
                                                    pass == 1 ? act_prev(pl.k) : nullptr,
                                                    pass == 1 ? act_items(pl.k) : nullptr);
             if (rc) return rc;
@@ -827,29 +701,6 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     CK(cudaMemsetAsync(ctx->d_count[1], 0, sizeof(int), s));
     CK(cudaMemsetAsync(ctx->d_stats, 0, 3 * sizeof(unsigned long long), s));
     CK(cudaMemsetAsync(ctx->d_trace, 0, 2 * sizeof(unsigned long long) * fm3dt_ctx::kTraceRounds, s));
-    // Certification of the events swept exactly once (all but the near-tie
-    // events, which had extra sweeps): their first round recomputes only the
-    // nodes it marks, on the tiles it appends to list 0
-    auto certify = [&](const int *events, int n, cudaStream_t st) {
-        auto fill = [&](auto &ca, const auto &f) {
-            ca.f = f;
-            ca.events = events; ca.nev = n;
-            ca.dir = ctx->d_dir;
-            ca.cert = ctx->d_cert; ca.cert_nw = ctx->cert_nw;
-            ca.tr = ts.tr; ca.tx = ts.tx; ca.tz = ts.tz;
-            ca.flag = ctx->d_flag; ca.list = ctx->d_list[0]; ca.count = ctx->d_count[0];
-        };
-        if (ctx->prec == FM3DT_FP64) {
-            CertifyArgs<double> ca{};
-            fill(ca, f64);
-            launch_certify_f64(ca, st);
-        } else {
-            CertifyArgs<float> ca{};
-            fill(ca, f32);
-            launch_certify_f32(ca, st);
-        }
-        ctx->launches += 1;
-    };
     const bool certify_alone = FM_CERTIFY && do_sweep && streaming && !verified && !overlap && !others.empty();
     if (!verified) {
         // (with the near-tie events' tiles queued by their last sweep, the
@@ -958,7 +809,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         CK(cudaEventCreate(&r1));
         CK(cudaMemcpyAsync(ev_buf, busy.data(), busy.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         CK(cudaEventRecord(r0, st));
-        const int rc = stream_pass((int)busy.size(), ev_buf, 0, 0, ctx->d_flag, list, count, st, false);
+        const int rc = stream_pass((int)busy.size(), ev_buf, 0, ctx->d_flag, list, count, st);
         if (rc) return rc;
         interval_nodes += (int64_t)busy.size() * (int64_t)ctx->N;
         CK(cudaEventRecord(r1, st));
@@ -1126,20 +977,20 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         }
         if (tie_queue) CK(cudaMemsetAsync(ctx->d_count_b, 0, sizeof(int), s2));
         CK(cudaEventRecord(pe[0], s2));
+        {
+            const int ra = act_start(s2);
+            if (ra) return ra;
+        }
         // the extra sweeps' own times (events between them on stream2)
         const int nts = std::min(ctx->tie_sweeps, fm3dt_ctx::kMaxTieSweeps);
         std::vector<cudaEvent_t> tse(nts + 1);
         for (auto &e : tse) CK(cudaEventCreate(&e));
         for (int k = 0; k < ctx->tie_sweeps; ++k) {
             if (k <= nts) CK(cudaEventRecord(tse[k], s2));
-            // (height segments by the time model for the near-tie events alone:
-            // their sweeps are the longer chain of the two parts); the last one
-            // queues their first round's tiles on list b
+            // (the last one queues their first round's tiles on list b)
             const bool q = tie_queue && k == ctx->tie_sweeps - 1;
-            const int rc = stream_pass((int)ties.size(), ctx->d_events, (k & 1) ? 0 : 4,
-                                       FM_OVERLAP_MAIN ? ctx->tie_segments : (ctx->tie_segments > 0 ? ctx->tie_segments : 2),
-                                       q ? ctx->d_flag : nullptr, ctx->d_list_b, ctx->d_count_b, s2, true,
-                                       act_cur(k), act_prev(k), act_items(k));
+            const int rc = stream_pass((int)ties.size(), ctx->d_events, (k & 1) ? 0 : 4, q ? ctx->d_flag : nullptr,
+                                       ctx->d_list_b, ctx->d_count_b, s2, act_cur(k), act_prev(k), act_items(k));
             if (rc) return rc;
         }
         if (ctx->tie_sweeps <= nts) CK(cudaEventRecord(tse[nts], s2));
@@ -1253,7 +1104,6 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         st->interval_nodes = interval_nodes;
     }
     if (kerr == 2) return fail(ctx, FM3DT_ECUDA, "a tile copy (TMA) destination was not 128-byte aligned");
-    if (kerr & 4) return fail(ctx, FM3DT_ECUDA, "a tracked sweep met an activity slot out of range");
     if (kerr & 16)
         return fail(ctx, FM3DT_ECUDA, "a sweep gave up waiting for upstream columns");
     if (kerr) return fail(ctx, FM3DT_ECUDA, "a tile copy (TMA) did not complete in time");
@@ -2288,8 +2138,7 @@ int fm3dt_set_sweep_segments(fm3dt_ctx *ctx, int segments, int tie_segments)
     if (!ctx) return FM3DT_EINVAL;
     if (segments < 0 || tie_segments < 0 || segments > 127 || tie_segments > 127)
         return fail(ctx, FM3DT_EINVAL, "segments outside 0..127");
-    ctx->sweep_segments = segments;
-    ctx->tie_segments = tie_segments;
+    // (the streaming sweeps take whole columns: any number gives the same sweep)
     return FM3DT_OK;
 }
 
@@ -2372,7 +2221,6 @@ void fm3dt_ctx_destroy(fm3dt_ctx *ctx)
 {
     if (!ctx) return;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (auto &sg : ctx->sweep_graphs) cudaGraphExecDestroy(sg.exec);
     for (auto e : ctx->round_events) cudaEventDestroy(e);
     for (auto e : ctx->round_events_b) cudaEventDestroy(e);
     cudaFree(ctx->d_velv);
@@ -2393,7 +2241,7 @@ void fm3dt_ctx_destroy(fm3dt_ctx *ctx)
     cudaFree(ctx->d_act_items);
     cudaFree(ctx->d_next);
     cudaFree(ctx->d_ray_events);
-    for (auto p : ctx->d_done) cudaFree(p);
+    for (auto p : ctx->d_prog) cudaFree(p);
     cudaFree(ctx->d_dense);
     cudaFree(ctx->d_compact);
     cudaFree(ctx->d_count_c);

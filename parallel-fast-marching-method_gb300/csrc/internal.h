@@ -89,9 +89,8 @@ struct SweepArgs {
     int nev;
 };
 
-// Streaming sweep (stream.cuh): one warp per column block of SX x SZ
-// columns streamed over the whole height; sweep shape indices kNumShapes and
-// up select these blocks.
+// Streaming sweeps (front.cuh, stream.cuh): one warp per column block of SX x
+// SZ columns; sweep shape indices kNumShapes and up select these blocks.
 struct StreamShape { int sx, sz; };
 constexpr int kNumStream = 2;
 constexpr StreamShape kStreamShapes[kNumStream] = {{4, 8}, {2, 16}};
@@ -100,46 +99,35 @@ constexpr int kNumSweepShapes = kNumShapes + kNumStream;
 template <typename R>
 struct StreamArgs {
     FieldArgs<R> f;
-    const int *hp_blocks;       // swept (segment, x block, z block): s << 24 | x' << 12 | z', by hyperplane
-    int hoff, hcount;
+    const int *blocks;          // swept column blocks x' << 12 | z', by hyperplane
+    int nblocks;
     const int *dir;             // [E] bit 0: sweep +theta, bit 1: sweep +phi, bits 2/3: near ties
     const int *events;          // the events swept (indices), or null for events 0..nev-1
     int nev;
+    int group;                  // events swept together (blocks are taken group by group)
     int flip;                   // bit 0 / 1: reverse theta / phi; bit 2: reverse each near-tie lateral direction
     int nbx, nbz;               // column blocks per axis
-    int seg_len;                // layers per height segment
-    // verification sweep: when flag is set, every node whose value changes
-    // queues its round tile (recompute all) and, near a tile face, the face
-    // neighbour (that face changed) -- the first round's work list
-    int *flag, *list, *count;
+    unsigned count;             // nblocks * nev
+    unsigned *next;             // blocks taken so far (zero at the start)
+    // per (event ordinal, block in grid order): layers final | chunks changed << 32
+    // (zero at the start)
+    unsigned long long *prog;
+    // when flag is set, every node whose value changes queues its round tile
+    // (recompute all) and, near a tile face, the face neighbour (that face
+    // changed) -- the next round's work list
+    int *flag, *list, *count_out;
     int tr, tx, tz;             // the rounds' tile shape and tile counts
     int ntr, ntx, ntz, tiles_per_event;
-    // activity (a chain of sweeps of the same events and height segments):
-    // per item (event ordinal, segment, column block in grid order) a mask of
-    // its chunks of 1 << act_shift layers in which a node changed in this
-    // sweep (act_cur) and in the previous one (act_prev).  A step of an item
-    // runs when one of its nodes lies in a chunk that can change: one near a
-    // chunk that changed in the previous sweep (in the item or a face
-    // neighbour), or earlier in this one (an upstream neighbour, or the item
-    // itself); act_cur null: no tracking, act_prev null: everything runs.
+    // activity (a chain of sweeps of the same events), slots as prog's: the
+    // chunks of 1 << act_shift layers in which a node changed in this sweep
+    // (act_cur; null: no tracking) and in the previous one (act_prev; null:
+    // every step runs)
     unsigned *act_cur;
     const unsigned *act_prev;
-    unsigned *act_run;          // the chunks of each item that run (stream_activity_kernel)
     int act_shift;
-    size_t act_n;               // masks in each activity buffer
-    int *err;                   // bit 2 raised: an activity slot out of range (not accessed)
-    // with tracking and a previous sweep (or null): [0] items that ran,
-    // [1] items skipped
+    // with a previous sweep (or null): [0] blocks that ran, [1] blocks passed by
     unsigned long long *act_items;
-    // one launch for the whole pass (flow): items taken in order from the
-    // counter *next (zero at the start), hp_blocks holding every hyperplane's
-    // blocks in order (hcount: all of them, hoff 0); an item starts when the
-    // done flags (zero at the start, done_n of them, same slots as the
-    // activity masks) of its three upstream neighbours are set
-    int flow;
-    unsigned *done;
-    size_t done_n;
-    unsigned *next;
+    int *err;                   // bit 4 raised: a wait for an upstream block gave up
 };
 
 // The main sweep (front.cuh): every listed event once, from a field filled
@@ -169,8 +157,8 @@ int occupancy_front_f64(int idx);
 
 void launch_stream_f32(int idx, int grid, const StreamArgs<float> &a, cudaStream_t st);
 void launch_stream_f64(int idx, int grid, const StreamArgs<double> &a, cudaStream_t st);
-int occupancy_stream_f32(int idx, bool flow);
-int occupancy_stream_f64(int idx, bool flow);
+int occupancy_stream_f32(int idx);
+int occupancy_stream_f64(int idx);
 
 // After a single sweep from an unset field: mark the nodes a recomputation
 // could change (certification bitmap) and queue their tiles (kCert).
@@ -184,6 +172,11 @@ struct CertifyArgs {
     int cert_nw;
     int tr, tx, tz;             // the rounds' tile shape
     int *flag, *list, *count;
+    // instead of the bitmap and the queue (or null): per (event ordinal, column
+    // block of bsx x bsz) the chunks of 1 << act_shift layers, counted from the
+    // bottom, that hold a marked node (zero at the start)
+    unsigned *act;
+    int act_shift, bsx, bsz, nbx, nbz;
 };
 void launch_certify_f32(const CertifyArgs<float> &a, cudaStream_t st);
 void launch_certify_f64(const CertifyArgs<double> &a, cudaStream_t st);
@@ -352,16 +345,14 @@ struct fm3dt_ctx {
     static constexpr int kTraceRounds = 8192;
     int last_rounds = 0;
     // tile hyperplanes of each shape (device list + host offsets)
-    struct Planes { int shape = -1; int nseg = 1; int *d_tiles = nullptr; std::vector<int> off, cnt; };
-    std::vector<Planes> block_planes;   // streaming sweeps, by (shape, height segments)
-    int sweep_segments = 0;       // height segments of the streaming sweep (0: automatic)
+    struct Planes { int shape = -1; int *d_tiles = nullptr; std::vector<int> off, cnt; };
+    std::vector<Planes> block_planes;   // streaming sweeps, by shape
     // solve schedule (fm3dt_set_schedule): extra sweeps of the near-tie events,
     // the near-tie band, re-sweeps after the first rounds and their threshold
     int tie_sweeps = 2;
     double tie_ratio = 0.1;
     int resweeps = 4;
     double resweep_frac = 0.01;
-    int tie_segments = 0;         // the same for the reversed sweep of near-tie events
     int *h_dir = nullptr;         // pinned [maxev] sweep directions of the last solve
     int *d_events = nullptr;      // [maxev] the near-tie events of the last solve
     // the first round of the other events runs on stream2 while the near-tie
@@ -375,15 +366,15 @@ struct fm3dt_ctx {
     int *d_count_c = nullptr;
     // item activity of the near-tie events' extra sweeps (this sweep's and
     // the previous one's, alternating), grown on demand
-    unsigned *d_act[3] = {nullptr, nullptr, nullptr};   // [2]: the chunks that run
+    unsigned *d_act[2] = {nullptr, nullptr};
     size_t act_bytes = 0;
     // items run / skipped by each of the last solve's near-tie extra sweeps
     static constexpr int kMaxTieSweeps = 16;
     unsigned long long *d_act_items = nullptr;   // [2 * kMaxTieSweeps]
-    // one-launch sweep passes: done flags and queue counters, per stream
-    // (context stream, stream2), the flags grown on demand
-    unsigned *d_done[2] = {nullptr, nullptr};
-    size_t done_bytes[2] = {0, 0};
+    // streaming sweeps: published words of their blocks, grown on demand, and
+    // block counters, per stream (context stream, stream2)
+    unsigned long long *d_prog[2] = {nullptr, nullptr};
+    size_t prog_bytes[2] = {0, 0};
     unsigned *d_next = nullptr;                  // [2]
     // the rays' dense rows and (host entry point) compacted rows, grown on demand
     float *d_dense = nullptr;
@@ -419,15 +410,6 @@ struct fm3dt_ctx {
     size_t flag_capacity = 0;     // tiles allocated for flags/lists
     int64_t launches = 0;
     std::string err;
-    // sweep passes captured as graphs, keyed by precision, sweep shape, event
-    // count, event list, flip, height segments, form, stream, tile shape,
-    // (flag mode) the flags and queue it writes, the activity it tracks and
-    // (one-launch passes) its done flags
-    static constexpr int kSweepKey = 15;
-    static constexpr size_t kSweepGraphs = 24;
-    struct SweepGraph { long long key[kSweepKey]; cudaGraphExec_t exec; };
-    std::vector<SweepGraph> sweep_graphs;
-    bool sweep_graph_off = false;
     std::vector<cudaEvent_t> round_events;   // start/stop pairs of round kernels
     std::vector<cudaEvent_t> round_events_b; // ... of a second part's rounds (stream2)
     std::vector<float> round_ms_trace;       // device time of each round of the last solve

@@ -55,10 +55,10 @@ void launch_stream_f32(int idx, int grid, const StreamArgs<float> &a, cudaStream
 #undef C_
 }
 
-int occupancy_stream_f32(int idx, bool flow)
+int occupancy_stream_f32(int idx)
 {
     int r = 0;
-#define C_(X, Z) r = StreamKernels<float, X, Z>::occ(flow)
+#define C_(X, Z) r = StreamKernels<float, X, Z>::occ()
     FM_STREAM_SWITCH(idx, C_)
 #undef C_
     return r;
