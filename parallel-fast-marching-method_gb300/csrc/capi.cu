@@ -313,7 +313,7 @@ void launch_ray_list(fm3dt_ctx *ctx, int nev, const fm3dt_ctx::EarlyRays &er, co
     ra.g = ctx->g;
     ra.prec = ctx->prec;
     ra.T = ctx->d_T;
-    ra.veln = ctx->d_veln;
+    ra.velf = ctx->d_velf;
     ra.nev = nev;
     ra.nrc = er.nrc;
     ra.events = d_events;
@@ -1210,6 +1210,7 @@ int fm3dt_ctx_create(const fm3dt_grid_desc *desc, fm3dt_ctx **out)
     const size_t npad = (size_t)(d.nnr + 3) * (d.nnx + 3) * (d.nnz + 3);
     CKC(cudaMalloc(&ctx->d_velv, nvel * sizeof(double)));
     CKC(cudaMalloc(&ctx->d_veln, npad * sizeof(double)));
+    CKC(cudaMalloc(&ctx->d_velf, npad * sizeof(float)));
     CKC(cudaMalloc(&ctx->d_s, ctx->N * rs));
     CKC(cudaMalloc(&ctx->d_hx, (size_t)d.nnr * rs));
     CKC(cudaMalloc(&ctx->d_hz, (size_t)d.nnr * d.nnx * rs));
@@ -1274,7 +1275,7 @@ int fm3dt_set_velocity(fm3dt_ctx *ctx, const double *velv)
     DeviceScratch sc(ctx);
     CK(sc.alloc(&d_sums, gridder_scratch(g)));
     CK(cudaMemcpyAsync(ctx->d_velv, velv, nvel * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    launch_gridder(g, ctx->d_velv, ctx->d_veln, ctx->d_s, ctx->prec, d_sums, ctx->stream);
+    launch_gridder(g, ctx->d_velv, ctx->d_veln, ctx->d_velf, ctx->d_s, ctx->prec, d_sums, ctx->stream);
     ctx->launches += 4;
     CKL();
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1411,7 +1412,7 @@ int fm3dt_solve_point(fm3dt_ctx *ctx, int nev, const double *src, int refine, in
             DeviceScratch sc(fc);
             double *d_sums = nullptr;
             CK(sc.alloc(&d_sums, gridder_scratch(fg)));
-            launch_gridder(fg, fc->d_velv, fc->d_veln, fc->d_s, fc->prec, d_sums, fc->stream);
+            launch_gridder(fg, fc->d_velv, fc->d_veln, fc->d_velf, fc->d_s, fc->prec, d_sums, fc->stream);
             fc->have_velocity = 1;
             // straight-ray start within two fine cells of the source
             int fb[6];
@@ -1538,7 +1539,7 @@ static int rays_trace(fm3dt_ctx *ctx, DeviceScratch &sc, int nrc, const double *
     ra.g = g;
     ra.prec = ctx->prec;
     ra.T = ctx->d_T;
-    ra.veln = ctx->d_veln;
+    ra.velf = ctx->d_velf;
     ra.nev = nev;
     ra.nrc = nrc;
     ra.rcr = d_rcr;
@@ -2225,6 +2226,7 @@ void fm3dt_ctx_destroy(fm3dt_ctx *ctx)
     for (auto e : ctx->round_events_b) cudaEventDestroy(e);
     cudaFree(ctx->d_velv);
     cudaFree(ctx->d_veln);
+    cudaFree(ctx->d_velf);
     cudaFree(ctx->d_s);
     cudaFree(ctx->d_hx);
     cudaFree(ctx->d_hz);

@@ -202,7 +202,7 @@ inline int sweep_blocks_per_sm(int shape, int prec)
 // padded velocity and interior slowness from the velocity nodes (four
 // launches); scratch: gridder_scratch(g) doubles
 size_t gridder_scratch(const Geom &g);
-void launch_gridder(const Geom &g, const double *velv, double *veln, void *s, int prec, double *scratch,
+void launch_gridder(const Geom &g, const double *velv, double *veln, float *velf, void *s, int prec, double *scratch,
                     cudaStream_t st);
 
 // boundary.cu
@@ -277,7 +277,7 @@ struct RayArgs {
     Geom g;
     int prec;
     const void *T;              // [E][N] traveltimes (R)
-    const double *veln;         // padded velocity (-1..n+1)
+    const float *velf;          // padded velocity (-1..n+1)
     int nev, nrc;
     const int *events;          // the events traced (nlist of them), or null for all nev
     int nlist;
@@ -311,6 +311,7 @@ struct fm3dt_ctx {
     // device buffers
     double *d_velv = nullptr;
     double *d_veln = nullptr;
+    float *d_velf = nullptr;      // the same in single precision
     void *d_s = nullptr;
     void *d_hx = nullptr;
     void *d_hz = nullptr;

@@ -109,10 +109,10 @@ __global__ void spline_x_kernel(Geom g, const SplineAxis *__restrict__ ax, const
 
 // sums over phi, one warp per (layer, row) of nodes; and the slowness
 // 1/velocity of the interior nodes (F:642), in the solver's precision, phi
-// fastest
+// fastest; velf: the velocity in single precision, for the rays' weights
 template <typename R>
 __global__ void spline_z_kernel(Geom g, const SplineAxis *__restrict__ ax, const double *__restrict__ xs,
-                                double *__restrict__ veln, R *__restrict__ s)
+                                double *__restrict__ veln, float *__restrict__ velf, R *__restrict__ s)
 {
     const int NVZ = g.nvz + 2, PX = g.nnx + 3, PZ = g.nnz + 3;
     const long long rows = (long long)(g.nnr + 3) * PX;
@@ -127,6 +127,7 @@ __global__ void spline_z_kernel(Geom g, const SplineAxis *__restrict__ ax, const
             double sum = 0.0;
             for (int i1 = 0; i1 < 4; ++i1) sum = sum + a.w[i1] * v[clampi((int)a.c + i1, 0, g.nvz + 1)];
             veln[(size_t)kj * PZ + i] = sum;
+            velf[(size_t)kj * PZ + i] = (float)sum;
             if (in && i >= 2 && i < g.nnz + 2) sr[i - 2] = (R)(1.0 / sum);
         }
     }
@@ -145,7 +146,7 @@ size_t gridder_scratch(const Geom &g)
     return axes + (size_t)(g.nnr + 3) * (g.nvz + 2) * ((g.nvx + 2) + (size_t)(g.nnx + 3));
 }
 
-void launch_gridder(const Geom &g, const double *velv, double *veln, void *s, int prec, double *scratch,
+void launch_gridder(const Geom &g, const double *velv, double *veln, float *velf, void *s, int prec, double *scratch,
                     cudaStream_t st)
 {
     const int na = g.nnr + g.nnx + g.nnz + 9;
@@ -159,9 +160,9 @@ void launch_gridder(const Geom &g, const double *velv, double *veln, void *s, in
     const dim3 block(32, 4);
     const int grid = grid_for((long long)(g.nnr + 3) * (g.nnx + 3), 4);
     if (prec == FM3DT_FP64)
-        spline_z_kernel<double><<<grid, block, 0, st>>>(g, ax, xs, veln, (double *)s);
+        spline_z_kernel<double><<<grid, block, 0, st>>>(g, ax, xs, veln, velf, (double *)s);
     else
-        spline_z_kernel<float><<<grid, block, 0, st>>>(g, ax, xs, veln, (float *)s);
+        spline_z_kernel<float><<<grid, block, 0, st>>>(g, ax, xs, veln, velf, (float *)s);
 }
 
 }  // namespace fm3dt
