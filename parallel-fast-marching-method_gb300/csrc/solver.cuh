@@ -293,6 +293,8 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
     __shared__ int s_face;
     __shared__ int s_w;
     __shared__ unsigned s_chg[2][TX * TZ];        // per column: nodes changed in a pass
+    __shared__ int s_nlist[2];                    // nodes a pass recomputes ...
+    __shared__ unsigned short s_list[TR * TX * TZ];   // ... and which (row * columns + column)
     __shared__ unsigned long long s_upd;
     const FieldArgs<R> &f = a.f;
     const int tid = threadIdx.x;
@@ -324,7 +326,9 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
             // activations re-queue it
             s_dirty_faces = atomicExch(&a.flag[w], 0) & (kFaceMask | kFull | kCert);
             __threadfence();
+            s_nlist[0] = s_nlist[1] = 0;
         }
+        s_chg[0][tid] = s_chg[1][tid] = 0;
         __syncthreads();
         const int w = s_w;
         const int e = w / f.tiles_per_event;
@@ -402,26 +406,65 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
                 dirty |= (a.cert[(((size_t)e * f.nnx + gx) * f.nnz + gz) * a.cert_nw + (r0 >> 5)] >> (r0 & 31)) & all;
             dirty &= updm;
         }
+        // A pass's nodes are spread over the threads: collected in a list, one
+        // a thread, unless there are more than two a thread; then each thread
+        // takes its own column's, in order (upward on even passes, downward on
+        // odd ones, which carries a value up or down a column in one pass).
+        // Far from the first pass a tile has a front of some tens of nodes to
+        // recompute, which a thread per column does one row after the other in
+        // mostly idle warps, each row the whole latency of an update (a pass of
+        // 4 to 8 rows is 3-5 us single, 20 us double precision).  Two
+        // double-precision events on 192x224x224 247 -> 192 ms (rounds 165 ->
+        // 115 ms), 32 on 128^3 26.6 -> 23.5 ms, a point source pair on 96^3
+        // 23.4 -> 20.2 ms.
         for (int p = 0; p < a.max_passes; ++p) {
-            unsigned pch = 0;
-            // r changes only shared-memory offsets and mask bits: no unrolling
-            const int k0 = (p & 1) ? 0 : TR - 1, dk = (p & 1) ? 1 : -1;
-            my_upd += __popc(dirty);
+            const int cnt = __popc(dirty);
+            my_upd += cnt;
+            int before = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, before, o);
+                if ((tid & 31) >= o) before += y;
+            }
+            int at = 0;
+            if ((tid & 31) == 31 && before) at = atomicAdd(&s_nlist[p & 1], before);
+            at = __shfl_sync(0xffffffffu, at, 31) + before - cnt;
+            for (unsigned m = dirty; m; m &= m - 1) s_list[at++] = (unsigned short)((__ffs(m) - 1) * TL::NT + tid);
+            __syncthreads();
+            // (the other parity's masks and count, last read before this
+            // barrier, next written after the one below)
+            s_chg[(p & 1) ^ 1][tid] = 0;
+            if (tid == 0) s_nlist[(p & 1) ^ 1] = 0;
+            const int n = s_nlist[p & 1];
+            const bool columns = n > 2 * TL::NT;
+            bool any = false;
 #pragma unroll 1
-            for (int i = 0, k = k0; i < TR; ++i, k += dk) {
-                if (!((dirty >> k) & 1u)) continue;
-                const int c = cbase + k * TL::SR;
-                const R nv = TL::update(box, c, f, k, tx, tz, r0 + k, gx, gz);
+            for (int i = 0;; ++i) {
+                int k, col = tid;
+                if (columns) {
+                    if (i >= TR) break;
+                    k = (p & 1) ? i : TR - 1 - i;
+                    if (!((dirty >> k) & 1u)) continue;
+                } else {
+                    const int j = i * TL::NT + tid;
+                    if (j >= n) break;
+                    k = s_list[j] / TL::NT;
+                    col = s_list[j] % TL::NT;
+                }
+                const int cx = col / TZ, cz = col % TZ;
+                const int c = ((2 + k) * TL::BX + (cx + 2)) * TL::BZ + (cz + TL::ZOFF);
+                const R nv = TL::update(box, c, f, k, cx, cz, r0 + k, x0 + cx, z0 + cz);
                 if (fbits(nv) != fbits(box[c])) {
                     box[c] = nv;
-                    pch |= 1u << k;
+                    atomicOr(&s_chg[p & 1][col], 1u << k);
+                    any = true;
                 }
             }
-            chm |= pch;
-            s_chg[p & 1][tid] = pch;
-            last_changed = __syncthreads_or(pch != 0) != 0;
-            if (!last_changed) break;
+            last_changed = __syncthreads_or(any) != 0;
             const unsigned *q = s_chg[p & 1];
+            const unsigned pch = q[tid];
+            chm |= pch;
+            if (!last_changed) break;
             unsigned lat = 0;
             if (tx > 0) lat |= q[tid - TZ];
             if (tx > 1) lat |= q[tid - 2 * TZ];
