@@ -41,7 +41,8 @@ __global__ void planewave_kernel(Geom g, PlaneWaveGeom pg, int nev, const double
 // (fixed nodes and their values) of the event's field.
 template <typename R>
 __global__ void finalize_kernel(Geom g, const double *__restrict__ frames, R *__restrict__ T,
-                                uint8_t *__restrict__ frozen, double *__restrict__ base, int offset_mode, R unset)
+                                uint8_t *__restrict__ frozen, double *__restrict__ base, double *__restrict__ first,
+                                int offset_mode, R unset)
 {
     const int e = blockIdx.x;
     const long long nb = (long long)g.nnx * g.nnz;
@@ -63,7 +64,10 @@ __global__ void finalize_kernel(Geom g, const double *__restrict__ frames, R *__
     }
     __syncthreads();
     const double b = (offset_mode && red[0] < DBL_MAX) ? red[0] : 0.0;
-    if (threadIdx.x == 0) base[e] = b;
+    if (threadIdx.x == 0) {
+        base[e] = b;
+        first[e] = red[0] < DBL_MAX ? red[0] - b : 0.0;
+    }
     R *bottom = T + (size_t)e * N + (size_t)(g.nnr - 1) * (size_t)nb;
     uint8_t *fz = frozen + (size_t)e * nb;
     for (long long q = threadIdx.x; q < nb; q += blockDim.x) {
@@ -170,7 +174,7 @@ void launch_planewave_frames(const Geom &g, const PlaneWaveGeom &pg, int nev, co
 }
 
 void launch_finalize_frames(const Geom &g, int nev, int prec, const double *frames, void *T, uint8_t *frozen,
-                            double *base, bool unwritten, cudaStream_t st)
+                            double *base, double *first, bool unwritten, cudaStream_t st)
 {
     double u64 = INFINITY;
     float u32 = INFINITY;
@@ -179,9 +183,9 @@ void launch_finalize_frames(const Geom &g, int nev, int prec, const double *fram
         memset(&u32, 0xff, sizeof u32);
     }
     if (prec == FM3DT_FP64)
-        finalize_kernel<double><<<nev, 512, 0, st>>>(g, frames, (double *)T, frozen, base, 0, u64);
+        finalize_kernel<double><<<nev, 512, 0, st>>>(g, frames, (double *)T, frozen, base, first, 0, u64);
     else
-        finalize_kernel<float><<<nev, 512, 0, st>>>(g, frames, (float *)T, frozen, base, 1, u32);
+        finalize_kernel<float><<<nev, 512, 0, st>>>(g, frames, (float *)T, frozen, base, first, 1, u32);
 }
 
 void launch_sweep_directions(const Geom &g, int nev, const double *frames, int *dir, double tie_ratio,

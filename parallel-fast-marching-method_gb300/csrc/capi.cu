@@ -353,7 +353,8 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
             CK(cudaMemsetAsync(ctx->d_T, 0xff, (size_t)nev * ctx->N * rsize(ctx->prec), s));
         else
             launch_fill_inf(ctx->d_T, (size_t)nev * ctx->N, ctx->prec, s);
-        launch_finalize_frames(g, nev, ctx->prec, ctx->d_frames, ctx->d_T, ctx->d_frozen, ctx->d_base, front, s);
+        launch_finalize_frames(g, nev, ctx->prec, ctx->d_frames, ctx->d_T, ctx->d_frozen, ctx->d_base,
+                               ctx->d_base + ctx->maxev, front, s);
         launch_sweep_directions(g, nev, ctx->d_frames, ctx->d_dir, ctx->tie_ratio, s);
         ctx->launches += 3;
         CKL();
@@ -734,13 +735,18 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
 
     const int bps = std::max(1, round_blocks_per_sm(shape, ctx->prec));
     const int grid = bps * sm_count();
-    const int max_rounds = ctx->max_rounds > 0 ? ctx->max_rounds : 64 * (ntr + ntx + ntz) + 256;
+    const int max_ordered = 2 * (g.nnr + g.nnx + g.nnz);   // rounds in the order of time, at most
+    const int max_rounds = ctx->max_rounds > 0 ? ctx->max_rounds : 64 * (ntr + ntx + ntz) + 256 + max_ordered;
     const int chunk = 8;
     RoundArgs<double> a64{};
     RoundArgs<float> a32{};
     a64.f = f64;
     a32.f = f32;
     a64.flag = a32.flag = ctx->d_flag;
+    a64.wake = a32.wake = ctx->d_wake;
+    a64.first = a32.first = mode == kPoint ? nullptr : ctx->d_base + ctx->maxev;
+    // (0: no tile is known to wait)
+    CK(cudaMemsetAsync(ctx->d_wake, 0, (size_t)nev * tpe * sizeof(unsigned), s));
     a64.max_passes = a32.max_passes = ctx->max_passes;
     a64.stats = a32.stats = ctx->d_stats;
     a64.err = a32.err = ctx->d_err;
@@ -755,6 +761,26 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         }
     }
 
+    // Rounds in the order of time (see RoundArgs::tau): the k-th keeps values
+    // above (k + 1) tau_step waiting.  The step is in units of the time a
+    // plane wave of any direction takes at most between neighbouring nodes'
+    // planes at the least velocity, (1/hr^2 + 1/hx^2 + 1/hz^2)^-1/2 / v.
+    // Point sources: from the first round on, three of them (two sources on
+    // 96^3, 5x refined: rounds as they come 20.2 ms; steps of 1.1, 1.6, 2.2,
+    // 2.7, 3.1, 3.7, 4.4 units 17.7, 14.1, 12.0, 11.3, 10.9, 10.9, 11.5 ms;
+    // seven more of 67^3 to 116^3, refined or not, alike).  Boundary frames:
+    // see decide, 2.5 (two events on 192x224x224 with 2, 2.5, 3, 3.9 units
+    // 112, 110, 123, 169 ms).  Not below half the mean node spacing along the
+    // grid's edges, so that a front crosses the grid in max_ordered rounds; what
+    // is later (boundary times of any range) comes unordered.  Only with the
+    // automatic round cap: a caller's cap counts rounds that come as before.
+    double tau_step = INFINITY;
+    if (ctx->max_rounds <= 0 && ctx->vmin > 0.0) {
+        const double r = g.earth + g.rgor, hr = g.dnr, hx = r * g.dnx, hz = r * g.dnz;
+        const double unit = 1.0 / std::sqrt(1.0 / (hr * hr) + 1.0 / (hx * hx) + 1.0 / (hz * hz));
+        const double edges = g.nnr * hr + g.nnx * hx + g.nnz * hz;
+        tau_step = std::max((mode == kPoint ? 3.0 : 2.5) * unit, edges / max_ordered) / ctx->vmin;
+    }
     int rounds = 0;
     bool done = false;
     double round_ms = 0.0, resweep_ms = 0.0;
@@ -767,9 +793,12 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     // it changes for the next round
     int resweeps_left = (do_sweep && streaming && !verified) ? ctx->resweeps : 0;
     int grid_override = 0;   // launch grid other than the persistent one (0: persistent)
-    auto launch_round = [&](int round, int *cur_list, int *cur_count, int *next_list, int *next_count,
+    // ordered: the count of rounds in the order of time before this one (-1: not so)
+    auto launch_round = [&](int round, int ordered, int *cur_list, int *cur_count, int *next_list, int *next_count,
                             cudaStream_t st) {
         const int gr = grid_override > 0 ? grid_override : grid;
+        a64.tau = ordered < 0 || ordered >= max_ordered ? INFINITY : (ordered + 1) * tau_step;
+        a32.tau = (float)a64.tau;
         if (ctx->prec == FM3DT_FP64) {
             a64.trace = round < fm3dt_ctx::kTraceRounds ? ctx->d_trace : nullptr;
             a64.round = round;
@@ -839,6 +868,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         cudaEvent_t ready;
         bool pending, done;
         int first, n;
+        int ordered;             // rounds in the order of time so far (-1: not in it)
     };
     auto part_launch = [&](Part &p) -> int {
         const int chunk_now = p.left > 0 ? 1 : chunk;
@@ -856,7 +886,8 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
             // tile, so blocks free up as they finish
             if (rounds == 0 && FM_ROUND0_PER_TILE && !verified && mode != kPoint && !certify_alone && !tie_queue)
                 grid_override = (int)std::min<long long>((long long)nev * cnt, 1LL << 30);
-            launch_round(rounds, p.L.list[cur], p.L.count[cur], p.L.list[nxt], p.L.count[nxt], p.st);
+            launch_round(rounds, p.ordered < 0 ? -1 : p.ordered++, p.L.list[cur], p.L.count[cur], p.L.list[nxt],
+                         p.L.count[nxt], p.st);
             grid_override = 0;
             CK(cudaEventRecord((*p.ev)[2 * k + 1], p.st));
             p.L.cur = nxt;
@@ -868,6 +899,22 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         p.pending = true;
         return FM3DT_OK;
     };
+    // Boundary frames in double precision are not swept again more than twice:
+    // if more tiles are left than CTAs are resident, the rounds go on in the
+    // order of time (fewer tiles take a round's latency whether or not they
+    // wait).  With the further re-sweeps and rounds as they come before: two
+    // events on 192x224x224 195 -> 136 ms, 39 on 44x84x61 51 -> 42, 12 on
+    // 53x110x64 31 -> 24, 49 on 183x61x108 87 -> 81; 17 on 185x81x75, 18 on
+    // 200x135x41 and 8 on 114x116x90 as before.  (Ordered without the two
+    // re-sweeps 195 -> 110, 51 -> 29 and 31 -> 18, but 87 -> 118, 72 -> 88 and
+    // 25 -> 30.  In single precision a round is cheap and a re-sweep more so: 63
+    // events on 202x89x85 17 -> 25.)
+    auto decide = [&](Part &p) {
+        if (ctx->max_rounds > 0 || mode != kFrames || ctx->prec != FM3DT_FP64) return;
+        if (p.left <= 0 || p.left > ctx->resweeps - 2) return;
+        p.left = 0;
+        if (*p.h_cnt > grid && (double)*p.h_cnt > ctx->resweep_frac * (double)nev * (double)tpe) p.ordered = 0;
+    };
     // (after the part's ready event) the chunk's times, re-sweeps, and the end
     auto part_finish = [&](Part &p) -> int {
         for (int q = 0; q < p.n; ++q) {
@@ -877,6 +924,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
             if ((int)ctx->round_ms_trace.size() < fm3dt_ctx::kTraceRounds) ctx->round_ms_trace.push_back(m);
         }
         p.pending = false;
+        decide(p);
         const int rc = maybe_resweep(p.st, p.h_cnt, p.L.list[p.L.cur], p.L.count[p.L.cur], *p.h_cnt, p.ev_buf, p.left);
         if (rc) return rc;
         if (*p.h_cnt == 0) p.done = true;
@@ -999,7 +1047,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
                                  ctx->d_flag, s2);
         CK(cudaEventRecord(pe[1], s2));
         CK(cudaMemsetAsync(ctx->d_count_c, 0, sizeof(int), s2));
-        launch_round(0, ctx->d_list_b, ctx->d_count_b, ctx->d_list_c, ctx->d_count_c, s2);
+        launch_round(0, -1, ctx->d_list_b, ctx->d_count_b, ctx->d_list_c, ctx->d_count_c, s2);
         CK(cudaEventRecord(pe[2], s2));
         CK(cudaEventRecord(join, s2));
         CK(cudaEventRecord(pe[3], s));
@@ -1009,13 +1057,13 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
             CK(cudaMemsetAsync(ctx->d_count[0], 0, sizeof(int), s));
             certify(ctx->d_events_b, (int)others.size(), s);
             CK(cudaEventRecord(pe[4], s));
-            launch_round(0, ctx->d_list[0], ctx->d_count[0], ctx->d_list[1], ctx->d_count[1], s);
+            launch_round(0, -1, ctx->d_list[0], ctx->d_count[0], ctx->d_list[1], ctx->d_count[1], s);
         } else {
             launch_initial_tiles((int)others.size(), ctx->d_events_b, tpe, first, cnt, ctx->d_list[0],
                                  ctx->d_count[0], ctx->d_flag, s);
             grid_override = (int)std::min<long long>((long long)others.size() * cnt, 1LL << 30);
             CK(cudaEventRecord(pe[4], s));
-            launch_round(0, ctx->d_list[0], ctx->d_count[0], ctx->d_list[1], ctx->d_count[1], s);
+            launch_round(0, -1, ctx->d_list[0], ctx->d_count[0], ctx->d_list[1], ctx->d_count[1], s);
             grid_override = 0;
         }
         CK(cudaEventRecord(pe[5], s));
@@ -1036,9 +1084,10 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         // at once).
         Part parts[2] = {
             {s, {{ctx->d_list[1], ctx->d_list[0]}, {ctx->d_count[1], ctx->d_count[0]}, 0}, ctx->d_events_b,
-             resweeps_left, ctx->h_count, &ctx->round_events, ready_ev[0], false, false, 0, 0},
+             resweeps_left, ctx->h_count, &ctx->round_events, ready_ev[0], false, false, 0, 0, -1},
             {s2, {{ctx->d_list_c, ctx->d_list_b}, {ctx->d_count_c, ctx->d_count_b}, 0}, ctx->d_events,
-             resweeps_left, ctx->h_count + 1, &ctx->round_events_b, ready_ev[1], false, false, 0, 0}};
+             resweeps_left, ctx->h_count + 1, &ctx->round_events_b, ready_ev[1], false, false, 0, 0, -1}};
+        decide(parts[0]);
         int rc = maybe_resweep(s, ctx->h_count, parts[0].L.list[0], parts[0].L.count[0], *ctx->h_count,
                                ctx->d_events_b, parts[0].left);
         if (rc) return rc;
@@ -1064,7 +1113,8 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         done = parts[0].done && parts[1].done;
     } else {
         Part part{s, {{ctx->d_list[0], ctx->d_list[1]}, {ctx->d_count[0], ctx->d_count[1]}, 0}, ctx->d_events,
-                  resweeps_left, ctx->h_count, &ctx->round_events, ready_ev[0], false, false, 0, 0};
+                  resweeps_left, ctx->h_count, &ctx->round_events, ready_ev[0], false, false, 0, 0,
+                  mode == kPoint && ctx->max_rounds <= 0 ? 0 : -1};
         const int rc = converge(&part, 1);
         if (rc) return rc;
         done = part.done;
@@ -1219,9 +1269,10 @@ int fm3dt_ctx_create(const fm3dt_grid_desc *desc, fm3dt_ctx **out)
     CKC(cudaMalloc(&ctx->d_dir, ctx->maxev * sizeof(int)));
     CKC(cudaMalloc(&ctx->d_T, ctx->N * ctx->maxev * rs));
     CKC(cudaMalloc(&ctx->d_frames, ctx->NB * ctx->maxev * sizeof(double)));
-    CKC(cudaMalloc(&ctx->d_base, ctx->maxev * sizeof(double)));
+    CKC(cudaMalloc(&ctx->d_base, 2 * (size_t)ctx->maxev * sizeof(double)));
     CKC(cudaMalloc(&ctx->d_frozen, ctx->NB * ctx->maxev));
     CKC(cudaMalloc(&ctx->d_flag, ctx->flag_capacity * sizeof(int)));
+    CKC(cudaMalloc(&ctx->d_wake, ctx->flag_capacity * sizeof(unsigned)));
     ctx->cert_nw = (d.nnr + 31) / 32;
     CKC(cudaMalloc(&ctx->d_cert, (size_t)ctx->maxev * d.nnx * d.nnz * ctx->cert_nw * sizeof(unsigned)));
     CKC(cudaMalloc(&ctx->d_list[0], ctx->flag_capacity * sizeof(int)));
@@ -1255,7 +1306,7 @@ int fm3dt_ctx_create(const fm3dt_grid_desc *desc, fm3dt_ctx **out)
         CKC(cudaStreamCreateWithPriority(&ctx->stream2, cudaStreamNonBlocking, greatest));
     }
     CKC(cudaMallocHost(&ctx->h_stats, 3 * sizeof(unsigned long long)));
-    CKC(cudaMemset(ctx->d_base, 0, ctx->maxev * sizeof(double)));
+    CKC(cudaMemset(ctx->d_base, 0, 2 * (size_t)ctx->maxev * sizeof(double)));
     int rc = ctx->prec == FM3DT_FP64 ? upload_geometry<double>(ctx) : upload_geometry<float>(ctx);
     if (rc != FM3DT_OK) return cleanup_fail(rc, ctx->err);
 #undef CKC
@@ -1271,6 +1322,7 @@ int fm3dt_set_velocity(fm3dt_ctx *ctx, const double *velv)
     for (size_t q = 0; q < nvel; ++q)
         if (!(velv[q] > 0.0) || !std::isfinite(velv[q]))
             return fail(ctx, FM3DT_EINVAL, "velocity values must be positive and finite");
+    const double vmin = *std::min_element(velv, velv + nvel);
     double *d_sums = nullptr;
     DeviceScratch sc(ctx);
     CK(sc.alloc(&d_sums, gridder_scratch(g)));
@@ -1280,6 +1332,7 @@ int fm3dt_set_velocity(fm3dt_ctx *ctx, const double *velv)
     CKL();
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->have_velocity = 1;
+    ctx->vmin = vmin;
     return FM3DT_OK;
 }
 
@@ -1414,6 +1467,7 @@ int fm3dt_solve_point(fm3dt_ctx *ctx, int nev, const double *src, int refine, in
             CK(sc.alloc(&d_sums, gridder_scratch(fg)));
             launch_gridder(fg, fc->d_velv, fc->d_veln, fc->d_velf, fc->d_s, fc->prec, d_sums, fc->stream);
             fc->have_velocity = 1;
+            fc->vmin = ctx->vmin;
             // straight-ray start within two fine cells of the source
             int fb[6];
             const double ff[3] = {(fg.rgor - ps[e].h) / fg.dnr, (ps[e].th - fg.rgox) / fg.dnx,
@@ -2256,6 +2310,7 @@ void fm3dt_ctx_destroy(fm3dt_ctx *ctx)
     cudaFree(ctx->d_base);
     cudaFree(ctx->d_frozen);
     cudaFree(ctx->d_flag);
+    cudaFree(ctx->d_wake);
     cudaFree(ctx->d_cert);
     cudaFree(ctx->d_list[0]);
     cudaFree(ctx->d_list[1]);

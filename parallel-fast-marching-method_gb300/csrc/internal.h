@@ -68,8 +68,17 @@ struct RoundArgs {
     int round;
     // nodes a certified tile recomputes first: bit r%32 of word
     // ((e*nnx + x)*nnz + z)*cert_nw + r/32 (or null)
-    const unsigned *cert;
+    unsigned *cert;
     int cert_nw;
+    // A round in the order of time: a node's new value above tau (+ the
+    // event's `first`) waits.  The node keeps its value, is marked in the
+    // bitmap, and its tile goes on to the next round's list -- where it is
+    // only passed on while all that waits in it is still above tau.  So a
+    // correction settles the nodes before it while it passes, instead of every
+    // intermediate value crossing the grid.  tau +inf: none waits.
+    R tau;
+    const double *first;        // [E] times that tau counts from (null: 0)
+    unsigned *wake;             // [E*tiles] no later than the earliest time that waits in the tile (float bits)
     // tile + halo box by one TMA copy (tma != 0): the field as a 4-D tensor
     // (phi, theta, r, event) with the box of the tile shape; err is raised if
     // a copy does not complete in time
@@ -212,7 +221,7 @@ void launch_planewave_frames(const Geom &g, const PlaneWaveGeom &pg, int nev, co
 // (unwritten: boundary nodes without a time get all ones, to be written by the
 // main sweep, instead of +inf)
 void launch_finalize_frames(const Geom &g, int nev, int prec, const double *frames, void *T,
-                            uint8_t *frozen, double *base, bool unwritten, cudaStream_t st);
+                            uint8_t *frozen, double *base, double *first, bool unwritten, cudaStream_t st);
 void launch_fill_inf(void *T, size_t n, int prec, cudaStream_t st);
 // n doubles between device memory and the device mapping of page-locked host
 // memory (either way round), by a kernel
@@ -334,6 +343,8 @@ struct fm3dt_ctx {
     std::vector<double> h_base;
     double hr = 0.0;
     int have_velocity = 0;
+    double vmin = 0.0;            // least velocity node
+    unsigned *d_wake = nullptr;   // [flag capacity] earliest time waiting in a tile
     int nev_solved = 0;
     // tuning
     int shape = 0;

@@ -276,6 +276,10 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, int phase)
         if (clock64() - t0 > kTmaWaitCycles) return false;
     }
 }
+// A waiting value rounded down to single precision, as ordered bits (times are
+// zero or above).
+__device__ __forceinline__ unsigned wake_bits(float v) { return __float_as_uint(v); }
+__device__ __forceinline__ unsigned wake_bits(double v) { return __float_as_uint(fm_narrow(v)); }
 template <typename R, int TR, int TX, int TZ>
 __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
     round_kernel(const __grid_constant__ RoundArgs<R> a)
@@ -293,6 +297,10 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
     __shared__ int s_face;
     __shared__ int s_w;
     __shared__ unsigned s_chg[2][TX * TZ];        // per column: nodes changed in a pass
+    __shared__ unsigned s_wait[TX * TZ];          // per column: nodes whose value is above tau
+    const bool waits = a.tau < Lim<R>::inf();     // a round in the order of time
+    __shared__ R s_tau;                           // the event's tau
+    __shared__ unsigned s_wake;                   // earliest value above it
     __shared__ int s_nlist[2];                    // nodes a pass recomputes ...
     __shared__ unsigned short s_list[TR * TX * TZ];   // ... and which (row * columns + column)
     __shared__ unsigned long long s_upd;
@@ -321,16 +329,32 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
         if (tid == 0) {
             const int w = a.cur_list[item];
             s_w = w;
+            s_wake = 0x7f800000u;
+            if (waits) {
+                const int ev = w / f.tiles_per_event;
+                s_tau = a.tau + (a.first ? (R)a.first[ev] : R(0));
+                const int fl = __ldcg(a.flag + w);
+                if (!(fl & (kFaceMask | kFull)) && (R)__uint_as_float(__ldcg(a.wake + w)) > s_tau) {
+                    // nothing but nodes that wait longer: on to the next round
+                    a.next_list[atomicAdd(a.next_count, 1)] = w;
+                    s_w = -1;
+                }
+            }
             s_face = 0;
             // take the halo faces changed since this tile's last pass; later
             // activations re-queue it
-            s_dirty_faces = atomicExch(&a.flag[w], 0) & (kFaceMask | kFull | kCert);
+            if (s_w >= 0) s_dirty_faces = atomicExch(&a.flag[w], 0) & (kFaceMask | kFull | kCert);
             __threadfence();
             s_nlist[0] = s_nlist[1] = 0;
         }
-        s_chg[0][tid] = s_chg[1][tid] = 0;
+        s_chg[0][tid] = s_chg[1][tid] = s_wait[tid] = 0;
         __syncthreads();
         const int w = s_w;
+        if (w < 0) {
+            __syncthreads();
+            continue;
+        }
+        const R tau = waits ? s_tau : Lim<R>::inf();
         const int e = w / f.tiles_per_event;
         const int t = w - e * f.tiles_per_event;
         const int tzi = t % f.ntz;
@@ -403,7 +427,8 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
             // could change (TR divides 32, so a column's rows of the tile lie
             // in one bitmap word)
             if ((df & kCert) && colv)
-                dirty |= (a.cert[(((size_t)e * f.nnx + gx) * f.nnz + gz) * a.cert_nw + (r0 >> 5)] >> (r0 & 31)) & all;
+                dirty |= (__ldcg(a.cert + (((size_t)e * f.nnx + gx) * f.nnz + gz) * a.cert_nw + (r0 >> 5)) >> (r0 & 31)) &
+                         all;
             dirty &= updm;
         }
         // A pass's nodes are spread over the threads: collected in a list, one
@@ -455,9 +480,14 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
                 const int c = ((2 + k) * TL::BX + (cx + 2)) * TL::BZ + (cz + TL::ZOFF);
                 const R nv = TL::update(box, c, f, k, cx, cz, r0 + k, x0 + cx, z0 + cz);
                 if (fbits(nv) != fbits(box[c])) {
-                    box[c] = nv;
-                    atomicOr(&s_chg[p & 1][col], 1u << k);
-                    any = true;
+                    if (nv > tau && nv < Lim<R>::inf()) {
+                        atomicOr(&s_wait[col], 1u << k);
+                        atomicMin(&s_wake, wake_bits(nv));
+                    } else {
+                        box[c] = nv;
+                        atomicOr(&s_chg[p & 1][col], 1u << k);
+                        any = true;
+                    }
                 }
             }
             last_changed = __syncthreads_or(any) != 0;
@@ -490,9 +520,22 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
         if (chm && tz < 2) fb |= 16;
         if (chm && tz >= TZ - 2) fb |= 32;
         if (fb) atomicOr(&s_face, fb);
+        if (waits) {
+            // the nodes that wait: the tile's bits of the column's word (other
+            // tiles' bits of it are theirs to write)
+            const unsigned wait = s_wait[tid];
+            if (colv) {
+                constexpr unsigned all = (TR >= 32) ? 0xffffffffu : ((1u << TR) - 1u);
+                unsigned *word = a.cert + (((size_t)e * f.nnx + gx) * f.nnz + gz) * a.cert_nw + (r0 >> 5);
+                atomicAnd(word, ~(all << (r0 & 31)));
+                if (wait) atomicOr(word, wait << (r0 & 31));
+            }
+            if (wait) atomicOr(&s_face, 128);
+            if (tid == 0) a.wake[w] = s_wake;
+        }
         __threadfence();
         __syncthreads();
-        if (tid < 7) {
+        if (tid < 8) {
             int fl = s_face;
             if (tid == 6 && last_changed) fl |= 64;   // pass cap hit: run again
             if ((fl >> tid) & 1) {
@@ -506,7 +549,8 @@ __global__ void __launch_bounds__(TX * TZ, (MinBlocks<R, TX * TZ>::round))
                     case 3: nb = txi < f.ntx - 1 ? w + f.ntz : -1; bit = kFaceXm; break;
                     case 4: nb = tzi > 0 ? w - 1 : -1; bit = kFaceZp; break;
                     case 5: nb = tzi < f.ntz - 1 ? w + 1 : -1; bit = kFaceZm; break;
-                    default: nb = w; bit = kFull; break;
+                    case 6: nb = w; bit = kFull; break;
+                    default: nb = w; bit = kCert; break;
                 }
                 if (nb >= 0 && !(atomicOr(&a.flag[nb], bit | kQueued) & kQueued)) {
                     const int pos = atomicAdd(a.next_count, 1);
