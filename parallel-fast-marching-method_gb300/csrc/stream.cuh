@@ -16,7 +16,7 @@
 //
 // A sweep is one launch.  Warps take blocks from a counter, group of events by
 // group and hyperplane by hyperplane; a block follows the two upstream of it
-// layer by layer: each publishes, every kPublish layers, a word with the layers
+// layer by layer: each publishes, every layer or two, a word with the layers
 // it has finished and the chunks of layers it has changed (a release store),
 // and reads the halo of a layer only when both upstream words say it is final
 // (an acquire load; the halo columns come from L2).  The blocks a block waits
@@ -79,8 +79,13 @@ __device__ void stream_mark(const StreamArgs<R> &a, int e, int gr, int gx, int g
 // Polls of an upstream word (an L2 round trip and a short sleep each, about a
 // second in all) before the error flag is raised and the block goes on.
 constexpr unsigned kRelayPolls = 1u << 20;
-// Layers between two publications of a block's word (a fence each).
-constexpr int kPublish = 4;
+// Layers between two publications of a block's word.  Each costs a fence, and
+// delays the blocks downstream by as many steps each.  A step in double precision
+// is long against a fence: 1 (32 events on 128^3 with 1, 2, 4, 8, 16 layers 22.8,
+// 23.1, 23.6, 24.7, 26.9 ms; two on 192x224x224 130.5, 132.5, 134.5, 141, 152).
+// Single precision: 2 (500 events on 192x224x224 with 1, 2, 3, 4, 8 layers 95.1,
+// 94.5, 94.7, 94.9, 96.5 ms, three requests on 97^3 0.87, 0.87, 0.88, 0.89, 0.92).
+template <typename R> constexpr int kPublish = sizeof(R) == 8 ? 1 : 2;
 // Quiet steps ahead that are worth the reload of the rings.
 constexpr int kRelayJump = 6;
 
@@ -414,7 +419,7 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
                 dirty = dirty || __any_sync(0xffffffffu, changed);
             }
             ++t;
-            if (t - LAG >= published + kPublish && t < steps) publish(t - LAG);
+            if (t - LAG >= published + kPublish<R> && t < steps) publish(t - LAG);
         }
         if (lane == 0) {
             if (track) a.act_cur[slot] = chg;
