@@ -74,7 +74,7 @@ def parse():
     ap.add_argument("--sweep-mode", type=int, default=1,
                     help="with --shape: 1 sweep then rounds, 2 sweep + verifying sweep, 0 no sweep")
     ap.add_argument("--segments", type=int, nargs=2, default=(0, 0),
-                    help="streaming sweep height segments (all events, near-tie events); 0 = automatic")
+                    help="accepted without effect: the streaming sweeps take whole columns")
     ap.add_argument("--schedule", type=float, nargs=4, default=None,
                     metavar=("TIE_SWEEPS", "TIE_RATIO", "RESWEEPS", "RESWEEP_FRAC"),
                     help="with --shape: the solve schedule (negative keeps the default); without --shape the "
@@ -173,21 +173,19 @@ def measured_peak_hbm():
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per node of
 # each single-precision solver kernel, from ncu captures of smaller cases of
 # the same kernels: a first round with every tile staged (96^3, 64 events)
-# and a full mid-sweep launch of a main sweep (the upstream-only form) in four
-# height segments (128^3, 64 events: 118.1 MB over 3.87 M nodes); the bench
-# scales it to its own launches by the nodes they process.
-KERNEL_DRAM_BYTES_PER_NODE = {"round_kernel": 4.15, "stream_sweep_kernel": 30.5}
+# and the main sweep of 124 events on 128^3 (4,166 MB over 260 M nodes); the
+# bench scales it to its own launches by the nodes they process.
+KERNEL_DRAM_BYTES_PER_NODE = {"round_kernel": 4.15, "front_kernel": 16.0}
 
 # Warp instructions per node of the same kernels, from ncu's
-# smsp__inst_executed.sum: for the sweep, the same mid-sweep launch of a main
-# sweep (58.9 M over 3.87 M nodes; the sweep interval the roofline line times
-# holds the main sweeps and the re-sweeps, and the main sweeps are most of
-# it), and per node staged by the rounds on the 96^3 case (64 events: first
-# rounds after certification and tail rounds together, summed over every
-# launch of three solves).  The kernels are bound by instruction issue, so
-# the bench also reports the issue rate they reach against the SMs' peak of
-# four warp instructions per cycle.
-KERNEL_WARP_INST_PER_NODE = {"round_kernel": 41.6, "stream_sweep_kernel": 15.2}
+# smsp__inst_executed.sum: for the main sweep the same launch (2,464 M over
+# 260 M nodes; the sweep interval the roofline line times also holds the
+# re-sweeps, whose full update takes more), and per node staged by the rounds on
+# the 96^3 case (64 events: first rounds after certification and tail rounds
+# together, summed over every launch of three solves).  The kernels are bound
+# by instruction issue, so the bench also reports the issue rate they reach
+# against the SMs' peak of four warp instructions per cycle.
+KERNEL_WARP_INST_PER_NODE = {"round_kernel": 41.6, "front_kernel": 9.5}
 
 
 def workload_config(cfg, step, h, nev, nrc, prec):
@@ -520,7 +518,7 @@ def run_ours(a):
     # re-sweeps (the near-tie events' extra sweeps fall in the rounds' interval
     # when the batch is solved in two parts)
     main_nodes = sum(s["interval_nodes"] for s in sts)
-    sweep_name = "stream_sweep_kernel" if sweep_shape_dims[0] == "stream" else "sweep_kernel"
+    sweep_name = "front_kernel" if sweep_shape_dims[0] == "stream" else "sweep_kernel"
     # name: (interval ms, nodes in it, launches, nodes of all launches)
     kernels = {
         "round_kernel": (round_ms, staged, round_launches, staged),

@@ -267,8 +267,9 @@ int fm3dt_set_tuning(fm3dt_ctx *ctx, int tile_shape, int max_passes, int max_rou
  * near-tie events, alternating reversed and forward (0..16, default 2); the
  * near-tie band, a lateral component below tie_ratio times the other (0..1,
  * default 0.1: within ~6 degrees of an axis); re-sweeps after the first rounds
- * (0..16, default 4) of the events with more than resweep_frac of their tiles
- * still queued (default 0.01).  None of these changes the converged field;
+ * (0..16, default 4; double precision with the automatic round cap stops after
+ * two) of the events with more than resweep_frac of their tiles still queued
+ * (default 0.01).  None of these changes the converged field;
  * the best values depend on the model's heterogeneity. */
 int fm3dt_set_schedule(fm3dt_ctx *ctx, int tie_sweeps, double tie_ratio, int resweeps, double resweep_frac);
 
@@ -279,13 +280,10 @@ int fm3dt_set_schedule(fm3dt_ctx *ctx, int tie_sweeps, double tie_ratio, int res
  * changes the converged field. */
 int fm3dt_set_sweep_shape(fm3dt_ctx *ctx, int tile_shape);
 
-/* Height segments of the streaming sweep (its work items are column blocks
- * of one segment; more segments give more parallel items per launch and a
- * longer pipeline ramp), for the sweep of every event and for the two extra
- * sweeps of the events whose lateral direction is a near tie (within ~6
- * degrees of an axis).  0 = automatic: chosen from the batch size for the
- * main sweep, two segments for the extra sweeps (they run beside the other
- * events' first round). */
+/* Accepted for callers of earlier versions, and checked as before (counts
+ * outside 0..127 are refused), but without effect: a streaming sweep is one
+ * launch whose column blocks run over the whole height and follow each other
+ * layer by layer, so there are no height segments to choose. */
 int fm3dt_set_sweep_segments(fm3dt_ctx *ctx, int segments, int tie_segments);
 
 /* Per-round trace of the last solve: tiles processed and node updates of
@@ -309,8 +307,7 @@ int fm3dt_part_ms(fm3dt_ctx *ctx, float *ms);
 int fm3dt_rays_ms(fm3dt_ctx *ctx, float *ms);
 
 /* The last solve's near-tie extra sweeps after the first skip the work items
- * (a height segment of a block of columns of one event) where nothing near
- * them changed: run[k] / skipped[k] the items extra sweep k ran and skipped,
+ * (a block of columns of one event) where nothing near them changed: run[k] / skipped[k] the items extra sweep k ran and skipped,
  * for up to cap sweeps (sweep 0 runs every item and counts none).  Returns
  * the number of extra sweeps recorded (0 when none tracked activity). */
 int fm3dt_tie_sweep_items(fm3dt_ctx *ctx, int cap, int64_t *run, int64_t *skipped);

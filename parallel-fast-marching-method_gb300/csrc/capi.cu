@@ -563,9 +563,8 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     ctx->act_sweeps = 0;
     ctx->tie_sweep_n = 0;
     if (do_sweep && streaming) {
-        // streaming sweep: one launch per column-block hyperplane
-        // the events whose lateral direction is a near tie get two more
-        // sweeps, reversed and then forward
+        // streaming sweep, one launch; the events whose lateral direction is a
+        // near tie get more, reversed and forward in turn
         CK(cudaMemcpyAsync(ctx->h_dir, ctx->d_dir, nev * sizeof(int), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         bool holes = false;

@@ -6,8 +6,8 @@ streaming),
 shape also fixes the CTA size: one thread per column), (3) the solve
 schedule -- how many extra sweeps, alternately reversed and forward, the
 near-tie events get and how wide the near-tie band is -- and (4) the height
-segments of those sweeps (automatic, or a few more, whose smaller items skip
-more where nothing changed), keeping the fastest device time.  The schedule depends most on the model: on a smooth one
+segments setting, which the sweeps no longer use (all choices time alike), keeping
+the fastest device time.  The schedule depends most on the model: on a smooth one
 (Gaussian node noise) two extra sweeps of the events within ~6 degrees of an
 axis are best; on a checkerboard, whose fast cells carry head waves across
 the sweep direction, five or six of them over a band twice as wide halve the
@@ -23,7 +23,7 @@ from . import sweep_shapes, tile_shapes
 PASS_CAPS = (16, 64)
 # (extra sweeps of the near-tie events, near-tie band)
 SCHEDULES = ((2, 0.1), (3, 0.15), (4, 0.15), (5, 0.15), (5, 0.2), (6, 0.2), (8, 0.2), (10, 0.2))
-# height segments of the near-tie events' sweeps (0: the solver's time model)
+# height segments of the near-tie events' sweeps (accepted without effect)
 TIE_SEGMENTS = (0, 4, 8)
 
 
