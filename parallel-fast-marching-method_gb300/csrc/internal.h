@@ -118,8 +118,8 @@ struct StreamArgs {
     int nbx, nbz;               // column blocks per axis
     unsigned count;             // nblocks * nev
     unsigned *next;             // blocks taken so far (zero at the start)
-    // per (event ordinal, block in grid order): layers final | chunks changed << 32
-    // (zero at the start)
+    // per (event ordinal, block in grid order): steps made (bit 31: passed by) |
+    // chunks changed << 32 (zero at the start)
     unsigned long long *prog;
     // when flag is set, every node whose value changes queues its round tile
     // (recompute all) and, near a tile face, the face neighbour (that face

@@ -16,12 +16,12 @@
 //
 // A sweep is one launch.  Warps take blocks from a counter, group of events by
 // group and hyperplane by hyperplane; a block follows the two upstream of it
-// layer by layer: each publishes, every layer or two, a word with the layers
-// it has finished and the chunks of layers it has changed (a release store),
-// and reads the halo of a layer only when both upstream words say it is final
-// (an acquire load; the halo columns come from L2).  The blocks a block waits
-// for were taken before it by warps that run, so every wait ends; it is
-// bounded all the same.
+// step by step: each publishes, every step or two, a word with the steps it has
+// made and the chunks of layers it has changed (a release store), and a block
+// reads the halo of a step -- each column at the layer of the lane beside it --
+// only when both upstream words say it is final (an acquire load; the halo
+// columns come from L2).  The blocks a block waits for were taken before it by
+// warps that run, so every wait ends; it is bounded all the same.
 //
 // Tracked sweeps (the near-tie chain) run only where something can change: a
 // node is recomputed to the same bits unless a stencil neighbour changed since
@@ -34,10 +34,12 @@
 // published word tells before the step.  Quiet chunks are passed by without
 // loading them.
 //
-// Before, each hyperplane of blocks (in height segments) was a launch, or a
-// block waited for the whole segments upstream: the critical path was
-// hyperplanes x segment steps.  Now it is nnr + ~20 (blocks along theta + phi)
-// steps.
+// What bounds it is the chain: nnr steps and a block's lag for every hyperplane
+// of blocks, SX steps along theta and SZ along phi (and the publication's).
+// With whole layers instead of steps in the words, a block lagged SX + SZ - 1
+// steps along either: two double-precision events on 192x224x224 131 -> 120.5 ms,
+// 32 on 128^3 22.9 -> 21.4, 500 single-precision ones on 192x224x224 94.5 ->
+// 93.3, three requests on 97^3 0.87 -> 0.85.
 #pragma once
 #include "solver.cuh"
 
@@ -79,13 +81,15 @@ __device__ void stream_mark(const StreamArgs<R> &a, int e, int gr, int gx, int g
 // Polls of an upstream word (an L2 round trip and a short sleep each, about a
 // second in all) before the error flag is raised and the block goes on.
 constexpr unsigned kRelayPolls = 1u << 20;
-// Layers between two publications of a block's word.  Each costs a fence, and
+// Steps between two publications of a block's word.  Each costs a fence, and
 // delays the blocks downstream by as many steps each.  A step in double precision
-// is long against a fence: 1 (32 events on 128^3 with 1, 2, 4, 8, 16 layers 22.8,
-// 23.1, 23.6, 24.7, 26.9 ms; two on 192x224x224 130.5, 132.5, 134.5, 141, 152).
-// Single precision: 2 (500 events on 192x224x224 with 1, 2, 3, 4, 8 layers 95.1,
-// 94.5, 94.7, 94.9, 96.5 ms, three requests on 97^3 0.87, 0.87, 0.88, 0.89, 0.92).
+// is long against a fence: 1 (two events on 192x224x224 with 1, 2, 3 steps 120.5,
+// 122.3, 123.6 ms).  Single precision: 2 (500 events on 192x224x224 with 1, 2, 3
+// steps 94.1, 93.4, 93.5 ms).
 template <typename R> constexpr int kPublish = sizeof(R) == 8 ? 1 : 2;
+// In a block's word: the steps it tells of were passed by, so that the layers
+// below are final (a running block is LAG layers behind its leading lane).
+constexpr unsigned kPassed = 1u << 31;
 // Quiet steps ahead that are worth the reload of the rings.
 constexpr int kRelayJump = 6;
 
@@ -164,6 +168,7 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
         // this lane's halo columns (upstream, downstream) in the bottom layer
         const R *up[PU], *dn[PD];
         long long ustep[PU];
+        int late[PU];                                // steps after which a halo column is taken
         bool uok[PU], dok[PD];
 #pragma unroll
         for (int j = 0; j < PU; ++j) {
@@ -179,6 +184,7 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
             }
             uok[j] = q < NU && hx >= 0 && hx < f.nnx && hz >= 0 && hz < f.nnz;
             ustep[j] = q < NF ? layer : f.nnx;
+            late[j] = q < 2 * SZ ? q % SZ : q < NF ? (q - 2 * SZ) % SX : 0;
             up[j] = q < NF ? Tb : (q < NF + SX ? f.hz : f.wz) + (long long)(nnr - 1) * f.nnx;
             if (uok[j]) up[j] += q < NF ? (long long)hx * f.nnz + hz : hx;
         }
@@ -203,20 +209,27 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
         const unsigned long long *upw = nullptr;
         if (lane == 0 && bxp > 0) upw = a.prog + ((size_t)k * a.nbx + (sx ? bx - 1 : bx + 1)) * a.nbz + bz;
         if (lane == 1 && bzp > 0) upw = a.prog + ((size_t)k * a.nbx + bx) * a.nbz + (sz ? bz - 1 : bz + 1);
-        int avail = bxp > 0 || bzp > 0 ? 0 : nnr;    // layers final upstream
+        const int steps = nnr + LAG;
+        const bool up0 = bxp > 0 || bzp > 0;
+        int avail = up0 ? 0 : nnr;                   // layers final upstream
+        int ready = up0 ? 0 : steps;                 // steps whose halo is final
         unsigned um = 0;                             // chunks changed upstream, as far as known
-        auto need = [&](int L) {
-            L = min(L, nnr);
+        // waits until L layers and step t's halo are final
+        auto need = [&](int L, int t) {
             unsigned polls = 0;
-            while (avail < L) {
-                const unsigned long long w = upw ? ld_acquire_u64(upw) : (unsigned long long)nnr;
-                avail = min(__shfl_sync(0xffffffffu, (int)(unsigned)w, 0), __shfl_sync(0xffffffffu, (int)(unsigned)w, 1));
+            while (avail < L || ready <= t) {
+                const unsigned long long w = upw ? ld_acquire_u64(upw) : (unsigned long long)(kPassed | (unsigned)steps);
+                const int n = (int)((unsigned)w & ~kPassed);
+                const int la = min(nnr, (unsigned)w & kPassed ? n : n - LAG), ra = n >= steps ? steps : n - (lane ? SZ : SX) + 1;
+                avail = max(avail, min(__shfl_sync(0xffffffffu, la, 0), __shfl_sync(0xffffffffu, la, 1)));
+                ready = max(ready, min(__shfl_sync(0xffffffffu, ra, 0), __shfl_sync(0xffffffffu, ra, 1)));
                 const unsigned m = (unsigned)(w >> 32);
                 um = __shfl_sync(0xffffffffu, m, 0) | __shfl_sync(0xffffffffu, m, 1);
-                if (avail >= L) break;
+                if (avail >= L && ready > t) break;
                 if (++polls > kRelayPolls || ((polls & 63u) == 0u && (*(volatile int *)a.err & 16))) {
                     if (lane == 0) atomicOr(a.err, 16);
                     avail = nnr;
+                    ready = steps;
                 }
                 __nanosleep(20);
             }
@@ -234,17 +247,20 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
             }
             act = __reduce_or_sync(0xffffffffu, m);
         }
-        R hu[PU];                                    // the next layer's upstream halo and spacings
+        R hu[PU];                                    // the next step's upstream halo, the next layer's spacings
         R v1 = INF, v2 = INF, Xp = INF, Zp = INF, u1 = INF, u2 = INF;
-        auto load_up = [&](int L) {
-            need(L + 1);
+        auto load_up = [&](int t) {
+            need(0, t);
 #pragma unroll
-            for (int j = 0; j < PU; ++j) hu[j] = uok[j] ? __ldcg(up[j] - L * ustep[j]) : INF;
+            for (int j = 0; j < PU; ++j) {
+                const int L = t - late[j];
+                hu[j] = uok[j] && L >= 0 && L < nnr ? __ldcg(up[j] - L * ustep[j]) : INF;
+            }
         };
-        auto store_up = [&](int L) {
+        auto store_up = [&](int t) {
 #pragma unroll
             for (int j = 0; j < PU; ++j)
-                if (lane + 32 * j < NU) s_up[L & (RING - 1)][lane + 32 * j] = hu[j];
+                if (lane + 32 * j < NU) s_up[t & (RING - 1)][lane + 32 * j] = hu[j];
         };
         auto copy_own = [&](int L) {
             if (L >= 0 && L < nnr && colv) cp_async_elem(&s_own[L & (RING - 1)][lane], Tb + own - L * layer);
@@ -269,22 +285,13 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
             for (int L = max(0, t - LAG + 2); L < t + AHEAD + 2; ++L) copy_own(L);
             for (int L = max(0, t - LAG); L < t + AHEAD; ++L) copy_rest(L);
             asm volatile("cp.async.commit_group;\n" ::: "memory");
-            need(t + 1);
-            // (several layers' loads in flight)
-            for (int L0 = max(0, t - LAG); L0 < min(t, nnr); L0 += 4) {
-                R b[4][PU];
+            // (the spacings' rows; a step's halo is its own)
+            for (int L = max(0, t - LAG); L < min(t, nnr); ++L)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < PU; ++j)
-                        b[i][j] = uok[j] && L0 + i < nnr ? __ldcg(up[j] - (L0 + i) * ustep[j]) : INF;
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < PU; ++j)
-                        if (L0 + i < t && lane + 32 * j < NU) s_up[(L0 + i) & (RING - 1)][lane + 32 * j] = b[i][j];
-            }
-            if (t < nnr) load_up(t);
+                for (int j = 0; j < PU; ++j)
+                    if (lane + 32 * j >= NF && lane + 32 * j < NU)
+                        s_up[L & (RING - 1)][lane + 32 * j] = uok[j] ? __ldg(up[j] - L * ustep[j]) : INF;
+            load_up(t);
             const int rp = t - delay;
             auto at = [&](int L, bool in, long long c) -> R {
                 return colv && in && L >= 0 && L < nnr ? __ldcg(Tb + c - L * layer) : INF;
@@ -300,10 +307,10 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
         };
         int published = 0;
         bool dirty = false;                          // values stored since the last publication
-        auto publish = [&](int done) {
+        auto publish = [&](int done, unsigned passed) {
             __syncwarp();
             if (lane == 0) {
-                const unsigned long long w = (unsigned long long)(unsigned)done | (unsigned long long)chg << 32;
+                const unsigned long long w = (unsigned long long)(passed | (unsigned)done) | (unsigned long long)chg << 32;
                 // (with nothing stored there is nothing to release)
                 if (dirty)
                     st_release_u64(a.prog + slot, w);
@@ -315,7 +322,6 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
         };
         bool seated = false, ran = false;
         int first = 0;                               // lowest layer of the current run of steps
-        const int steps = nnr + LAG;
         int t = 0;
         while (t < steps) {
             if (skip) {
@@ -325,7 +331,7 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
                     // or that upstream has not left (chunks above the leading
                     // one; with none, to the end)
                     const int c = t < nnr ? (t >> sh) + 1 : 32;
-                    if (t < nnr) need(min(nnr, c << sh));
+                    need(t < nnr ? min(nnr, c << sh) : nnr, -1);
                     if (!((act | um) & range)) {
                         const int known = avail >= nnr ? 32 : avail >> sh;
                         const unsigned above = c < 32 ? (act | um) & (~0u << c) : 0u;
@@ -334,7 +340,7 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
                         if (!seated || tn - t >= kRelayJump) {
                             seated = false;
                             t = tn;
-                            if (t < steps) publish(t);
+                            if (t < steps) publish(t, kPassed);
                             continue;
                         }
                     }
@@ -346,8 +352,8 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
                 first = t;
             }
             // step t: layer t's halo into its ring, layer t + 1's on its way
-            if (t < nnr) store_up(t);
-            if (t + 1 < nnr) load_up(t + 1);
+            store_up(t);
+            if (t + 1 < steps) load_up(t + 1);
             copy_own(t + AHEAD + 2);
             copy_rest(t + AHEAD);
             asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -369,12 +375,12 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
             t1[5] = __shfl_down_sync(0xffffffffu, u1, 1);
             t2[5] = __shfl_down_sync(0xffffffffu, u2, 2);
             if (xs == 0) {
-                t1[2] = s_up[row][zs];
-                t2[2] = s_up[row][SZ + zs];
+                t1[2] = s_up[t & (RING - 1)][zs];
+                t2[2] = s_up[t & (RING - 1)][SZ + zs];
             }
             if (zs == 0) {
-                t1[4] = s_up[row][2 * SZ + xs];
-                t2[4] = s_up[row][2 * SZ + SX + xs];
+                t1[4] = s_up[t & (RING - 1)][2 * SZ + xs];
+                t2[4] = s_up[t & (RING - 1)][2 * SZ + SX + xs];
             }
             if (xs == SX - 1) t1[3] = s_dn[row][zs];
             if (xs >= SX - 2) t2[3] = s_dn[row][(xs - (SX - 2)) * SZ + zs];
@@ -419,13 +425,13 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
                 dirty = dirty || __any_sync(0xffffffffu, changed);
             }
             ++t;
-            if (t - LAG >= published + kPublish<R> && t < steps) publish(t - LAG);
+            if (t >= published + kPublish<R> && t < steps) publish(t, 0u);
         }
         if (lane == 0) {
             if (track) a.act_cur[slot] = chg;
             if (skip && a.act_items) atomicAdd(a.act_items + (ran ? 0 : 1), 1ull);
         }
-        publish(nnr);
+        publish(steps, kPassed);
     }
 }
 
