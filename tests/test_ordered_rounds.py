@@ -42,23 +42,28 @@ def test_point_order(gpu_lib, orc, nn, refine, depth):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("frac", [0.0, 0.01])
-def test_frames_order(gpu_lib, orc, frac):
+@pytest.mark.parametrize("nev", [12, 40])
+def test_frames_order(gpu_lib, orc, nev):
+    """Double precision, every event near an axis or most of them off the axes."""
     import fm3dt
     from fm3dt import synth
     w = synth.config(1, scale=24, nev=1)
-    h = _header(w.header, (96, 97, 99))
+    h = _header(w.header, (64, 65, 67))
     g = orc.grid_from_header(h.nv, h.vorig, h.vstep, h.nn, h.norig, h.nstep, h.earth)
-    i = np.indices((h.nv[2] + 2, h.nv[1] + 2, h.nv[0] + 2)).sum(0) // 2 % 2
+    i = (np.indices((h.nv[2] + 2, h.nv[1] + 2, h.nv[0] + 2)) // 3).sum(0) % 2
     velv = w.velv * np.where(i, 1.05, 0.95).reshape(-1)
-    frames = np.stack([orc.planewave_frame(g, orc.planewave_params(g, 50.0, b)).reshape(h.nn[1:])
-                       for b in (96.0, 278.0, 6.0)])
-    got = []
+    baz = [90.0 * (e % 4) + (6.0 + 0.3 * e if e < 12 else 20.0 + 1.7 * (e - 12)) for e in range(nev)]
+    frames = np.stack([orc.planewave_frame(g, orc.planewave_params(g, 40.0 + e, b)).reshape(h.nn[1:])
+                       for e, b in enumerate(baz)])
+    got, rounds = [], []
     for cap in (0, 1000000):
-        with fm3dt.Solver(h, fom=1, max_events=3, precision=fm3dt.FP64) as s:
+        with fm3dt.Solver(h, fom=1, max_events=nev, precision=fm3dt.FP64) as s:
             s.set_tuning(0, max_rounds=cap)
-            s.set_schedule(tie_sweeps=0, resweeps=2, resweep_frac=frac)
+            s.set_schedule(tie_sweeps=0)
             s.set_velocity(velv)
             s.solve(frames)
-            got.append(np.stack([s.get_times(e) for e in range(3)]))
+            got.append(np.stack([s.get_times(e) for e in range(nev)]))
+            rounds.append(len(s.round_trace()[0]))
+    # (rounds in the order of time are more, and smaller)
+    assert rounds[0] > rounds[1]
     assert np.array_equal(*got)
