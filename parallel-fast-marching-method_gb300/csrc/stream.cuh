@@ -112,9 +112,12 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned l
 // Chunk c of a mask and the chunks above and below it.
 __device__ __forceinline__ unsigned chunk_spread(unsigned m) { return m | (m << 1) | (m >> 1); }
 
-// Resident one-warp CTAs the registers must allow: in single precision 20 (96
-// registers; 24 and 28, with spills, measured slower), in double precision 12.
-template <typename R> struct RelayBlocks { static constexpr int value = 20; };
+// Resident one-warp CTAs the registers must allow: in single precision 16 (128
+// registers, no spills; warps mostly follow each other, so a shorter step counts
+// for more than another warp).  500 events on 192x224x224 with 14, 16, 18, 20
+// resident 92.3, 92.4, 93.3, 93.3 ms, with +-5% contrast 200, 198.5, 208, 206.5;
+// three requests on 97^3 0.83, 0.82, 0.845, 0.86.  In double precision 12.
+template <typename R> struct RelayBlocks { static constexpr int value = 16; };
 template <> struct RelayBlocks<double> { static constexpr int value = 12; };
 
 template <typename R, int SX, int SZ>
