@@ -47,6 +47,7 @@
 // precision 32 events on 128^3 30.5 -> 9.0 ms, one on 64^3 3.4 -> 0.89 ms (both with
 // the screened update).
 #pragma once
+#include "halo_layers.h"
 #include "stream.cuh"
 
 namespace fm3dt {
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(32) front_kernel(FrontArgs<R> a)
         const int row = t & (RING - 1);
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            if (hok[j] && (SKEW ? (unsigned)(t - hlate[j]) < (unsigned)nnr : t < nnr))
+            if (hok[j] && halo_layer_in(t, hlate[j], nnr))
                 cp_async_elem(&s_halo[row][lane + 32 * j], hp[j]);
             hp[j] -= hstep[j];
         }
@@ -205,15 +206,20 @@ __global__ void __launch_bounds__(32) front_kernel(FrontArgs<R> a)
                 for (int j = 0; j < PER; ++j)
                     wait = wait || (hok[j] && hfield[j] && front_unwritten(halo[lane + 32 * j]));
                 if (!__any_sync(0xffffffffu, wait)) break;
-                if (++polls > kFrontPolls || ((polls & 63u) == 0u && (*(volatile int *)a.err & 16))) {
-                    if (lane == 0) atomicOr(a.err, 16);
-                    break;
-                }
-                // (hp stands AHEAD + 1 layers above)
+                const bool give_up = ++polls > kFrontPolls || ((polls & 63u) == 0u && (*(volatile int *)a.err & 16));
+                // (hp stands AHEAD + 1 layers above.  After another wait gave
+                // up, rows of layers above the grid, which are not copied
+                // anew, can hold unwritten values too: not polled)
 #pragma unroll
                 for (int j = 0; j < PER; ++j)
                     if (hok[j] && hfield[j] && front_unwritten(halo[lane + 32 * j]))
-                        halo[lane + 32 * j] = front_load(hp[j] + (AHEAD + 1) * hstep[j]);
+                        halo[lane + 32 * j] = give_up || !halo_layer_in(t, hlate[j], nnr)
+                                                  ? INF
+                                                  : front_load(hp[j] + (AHEAD + 1) * hstep[j]);
+                if (give_up) {
+                    if (lane == 0) atomicOr(a.err, 16);
+                    break;
+                }
             }
         }
         // (a ring holds more layers than a step reads, so that a lane one step
