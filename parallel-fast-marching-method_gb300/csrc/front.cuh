@@ -82,10 +82,6 @@ __device__ __forceinline__ void front_store(double *p, double v)
     asm volatile("st.relaxed.gpu.global.f64 [%0], %1;\n" ::"l"(p), "d"(v) : "memory");
 }
 
-// Polls of a halo value (an L2 round trip each, about a second in all) before
-// the error flag is raised and the block goes on.
-constexpr unsigned kFrontPolls = 1u << 20;
-
 template <typename R, int SX, int SZ, bool SKEW>
 __global__ void __launch_bounds__(32) front_kernel(FrontArgs<R> a)
 {
@@ -206,7 +202,7 @@ __global__ void __launch_bounds__(32) front_kernel(FrontArgs<R> a)
                 for (int j = 0; j < PER; ++j)
                     wait = wait || (hok[j] && hfield[j] && front_unwritten(halo[lane + 32 * j]));
                 if (!__any_sync(0xffffffffu, wait)) break;
-                const bool give_up = ++polls > kFrontPolls || ((polls & 63u) == 0u && (*(volatile int *)a.err & 16));
+                const bool give_up = wait_gives_up(++polls, a.err);
                 // (hp stands AHEAD + 1 layers above.  After another wait gave
                 // up, rows of layers above the grid, which are not copied
                 // anew, can hold unwritten values too: not polled)
@@ -216,10 +212,7 @@ __global__ void __launch_bounds__(32) front_kernel(FrontArgs<R> a)
                         halo[lane + 32 * j] = give_up || !halo_layer_in(t, hlate[j], nnr)
                                                   ? INF
                                                   : front_load(hp[j] + (AHEAD + 1) * hstep[j]);
-                if (give_up) {
-                    if (lane == 0) atomicOr(a.err, 16);
-                    break;
-                }
+                if (give_up) break;
             }
         }
         // (a ring holds more layers than a step reads, so that a lane one step

@@ -78,9 +78,25 @@ __device__ void stream_mark(const StreamArgs<R> &a, int e, int gr, int gx, int g
     if (zi >= a.tz - 2 && tk < a.ntz - 1) stream_queue(a, w + 1, kFaceZm);
 }
 
-// Polls of an upstream word (an L2 round trip and a short sleep each, about a
-// second in all) before the error flag is raised and the block goes on.
-constexpr unsigned kRelayPolls = 1u << 20;
+// Polls of a halo value or an upstream word (an L2 round trip each, about a
+// second in all; a multiple of 64) before the error flag is raised and the
+// block goes on.
+#ifndef FM_WAIT_POLLS
+#define FM_WAIT_POLLS (1u << 20)
+#endif
+
+// Whether a warp's wait ends unanswered after `polls` polls: its limit is
+// reached, or another wait's was, looked for every 64th poll.  The warp decides
+// as one (a vote): lanes that saw the error word change between their reads
+// would otherwise part, and wait for each other in the votes and shuffles ahead.
+__device__ __forceinline__ bool wait_gives_up(unsigned polls, int *err)
+{
+    static_assert(FM_WAIT_POLLS % 64 == 0, "looked at every 64th poll");
+    if (polls & 63u) return false;
+    if (!__any_sync(0xffffffffu, polls >= FM_WAIT_POLLS || (*(volatile int *)err & 16))) return false;
+    if ((threadIdx.x & 31) == 0) atomicOr(err, 16);
+    return true;
+}
 // Steps between two publications of a block's word.  Each costs a fence, and
 // delays the blocks downstream by as many steps each.  A step in double precision
 // is long against a fence: 1 (two events on 192x224x224 with 1, 2, 3 steps 120.5,
@@ -229,8 +245,7 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
                 const unsigned m = (unsigned)(w >> 32);
                 um = __shfl_sync(0xffffffffu, m, 0) | __shfl_sync(0xffffffffu, m, 1);
                 if (avail >= L && ready > t) break;
-                if (++polls > kRelayPolls || ((polls & 63u) == 0u && (*(volatile int *)a.err & 16))) {
-                    if (lane == 0) atomicOr(a.err, 16);
+                if (wait_gives_up(++polls, a.err)) {
                     avail = nnr;
                     ready = steps;
                 }
