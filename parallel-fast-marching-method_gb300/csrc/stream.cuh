@@ -356,6 +356,10 @@ __global__ void __launch_bounds__(32, RelayBlocks<R>::value) relay_kernel(Stream
                         const int to = min(above ? __ffs(above) - 1 : 32, max(c, known));
                         const int tn = (to << sh) < nnr ? to << sh : steps;
                         if (!seated || tn - t >= kRelayJump) {
+                            // (copies of the last steps may still be on their
+                            // way into the rings, which are filled anew: two
+                            // copies to one place come in no order)
+                            if (seated) asm volatile("cp.async.wait_all;\n" ::: "memory");
                             seated = false;
                             t = tn;
                             if (t < steps) publish(t, kPassed);
