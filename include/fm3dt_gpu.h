@@ -267,10 +267,12 @@ int fm3dt_set_tuning(fm3dt_ctx *ctx, int tile_shape, int max_passes, int max_rou
  * near-tie events, alternating reversed and forward (0..16, default 2); the
  * near-tie band, a lateral component below tie_ratio times the other (0..1,
  * default 0.1: within ~6 degrees of an axis); re-sweeps after the first rounds
- * (0..16, default 4; double precision with the automatic round cap stops after
- * two) of the events with more than resweep_frac of their tiles still queued
- * (default 0.01).  None of these changes the converged field;
- * the best values depend on the model's heterogeneity. */
+ * (0..16) of the events with more than resweep_frac of their tiles still queued
+ * (default 0.01).  Until a number of re-sweeps is set it is chosen: four, or, in
+ * double precision with the automatic round cap, two and then rounds in the
+ * order of time if many tiles are left; a number that is set is kept to.  None
+ * of these changes the converged field; the best values depend on the model's
+ * heterogeneity. */
 int fm3dt_set_schedule(fm3dt_ctx *ctx, int tie_sweeps, double tie_ratio, int resweeps, double resweep_frac);
 
 /* Shape of the directional sweep (independent of the rounds' shape): a tile

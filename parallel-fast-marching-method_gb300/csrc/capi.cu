@@ -898,8 +898,8 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
         p.pending = true;
         return FM3DT_OK;
     };
-    // Boundary frames in double precision are not swept again more than twice:
-    // if more tiles are left than CTAs are resident, the rounds go on in the
+    // Boundary frames in double precision are not swept again more than twice,
+    // unless the caller set a number of re-sweeps: if more tiles are left than CTAs are resident, the rounds go on in the
     // order of time (fewer tiles take a round's latency whether or not they
     // wait).  With the further re-sweeps and rounds as they come before: two
     // events on 192x224x224 195 -> 136 ms, 39 on 44x84x61 51 -> 42, 12 on
@@ -909,7 +909,7 @@ int solve_common(fm3dt_ctx *ctx, int nev, fm3dt_status *st, int mode = kFrames)
     // 25 -> 30.  In single precision a round is cheap and a re-sweep more so: 63
     // events on 202x89x85 17 -> 25.)
     auto decide = [&](Part &p) {
-        if (ctx->max_rounds > 0 || mode != kFrames || ctx->prec != FM3DT_FP64) return;
+        if (ctx->max_rounds > 0 || ctx->resweeps_set || mode != kFrames || ctx->prec != FM3DT_FP64) return;
         if (p.left <= 0 || p.left > ctx->resweeps - 2) return;
         p.left = 0;
         if (*p.h_cnt > grid && (double)*p.h_cnt > ctx->resweep_frac * (double)nev * (double)tpe) p.ordered = 0;
@@ -2173,7 +2173,10 @@ int fm3dt_set_schedule(fm3dt_ctx *ctx, int tie_sweeps, double tie_ratio, int res
         return fail(ctx, FM3DT_EINVAL, "schedule: tie_sweeps and resweeps <= 16, ratios <= 1");
     if (tie_sweeps >= 0) ctx->tie_sweeps = tie_sweeps;
     if (tie_ratio >= 0.0) ctx->tie_ratio = tie_ratio;
-    if (resweeps >= 0) ctx->resweeps = resweeps;
+    if (resweeps >= 0) {
+        ctx->resweeps = resweeps;
+        ctx->resweeps_set = true;
+    }
     if (resweep_frac >= 0.0) ctx->resweep_frac = resweep_frac;
     return FM3DT_OK;
 }

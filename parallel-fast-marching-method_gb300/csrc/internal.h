@@ -364,6 +364,7 @@ struct fm3dt_ctx {
     int tie_sweeps = 2;
     double tie_ratio = 0.1;
     int resweeps = 4;
+    bool resweeps_set = false;    // by the caller: kept to (else see solve_common's decide)
     double resweep_frac = 0.01;
     int *h_dir = nullptr;         // pinned [maxev] sweep directions of the last solve
     int *d_events = nullptr;      // [maxev] the near-tie events of the last solve
