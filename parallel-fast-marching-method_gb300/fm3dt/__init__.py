@@ -236,7 +236,11 @@ class Solver:
     def set_sweep_shape(self, shape: int):
         self._check(self._L.fm3dt_set_sweep_shape(self._ctx, int(shape)))
 
+    # (a sweep's column blocks run over the whole height)
+    takes_sweep_segments = False
+
     def set_sweep_segments(self, segments: int = 0, tie_segments: int = 0):
+        """Accepted without effect (outside 0..127 refused)."""
         self._check(self._L.fm3dt_set_sweep_segments(self._ctx, int(segments), int(tie_segments)))
 
     def round_trace(self, cap: int = 8192):

@@ -1,17 +1,16 @@
 """Autotuner of the tile solver.
 
 Tunes, on a sample batch, (1) the shape of the directional sweep (tile or
-streaming),
-(2) the tile shape and in-tile pass cap of the fast-iterative rounds (the
-shape also fixes the CTA size: one thread per column), (3) the solve
-schedule -- how many extra sweeps, alternately reversed and forward, the
-near-tie events get and how wide the near-tie band is -- and (4) the height
-segments setting, which the sweeps no longer use (all choices time alike), keeping
-the fastest device time.  The schedule depends most on the model: on a smooth one
-(Gaussian node noise) two extra sweeps of the events within ~6 degrees of an
-axis are best; on a checkerboard, whose fast cells carry head waves across
-the sweep direction, five or six of them over a band twice as wide halve the
-rounds.  The converged field does not depend on any of these choices (the
+streaming), (2) the tile shape and in-tile pass cap of the fast-iterative
+rounds (the shape also fixes the CTA size: one thread per column) and (3) the
+solve schedule -- how many extra sweeps, alternately reversed and forward, the
+near-tie events get and how wide the near-tie band is -- keeping the fastest
+device time.  (4) The height segments setting is timed only on a solver that
+takes one; ``fm3dt.Solver`` accepts it without effect.  The schedule depends
+most on the model: on a smooth one (Gaussian node noise) two extra sweeps of
+the events within ~6 degrees of an axis are best; on a checkerboard, whose fast
+cells carry head waves across the sweep direction, five or six of them over a
+band twice as wide halve the rounds.  The converged field does not depend on any of these choices (the
 fixed point is unique), so tuning never changes results.
 """
 from __future__ import annotations
@@ -23,7 +22,7 @@ from . import sweep_shapes, tile_shapes
 PASS_CAPS = (16, 64)
 # (extra sweeps of the near-tie events, near-tie band)
 SCHEDULES = ((2, 0.1), (3, 0.15), (4, 0.15), (5, 0.15), (5, 0.2), (6, 0.2), (8, 0.2), (10, 0.2))
-# height segments of the near-tie events' sweeps (accepted without effect)
+# height segments of the near-tie events' sweeps, on a solver that takes them
 TIE_SEGMENTS = (0, 4, 8)
 
 
@@ -37,7 +36,8 @@ def autotune(solver, frames_ptr: int, nev: int, device: bool = True, repeats: in
     """Returns (round_shape, max_passes, sweep_shape, ms, schedule,
     tie_segments) and applies it; schedule = (tie_sweeps, tie_ratio,
     resweeps, resweep_frac), negative values being the defaults kept;
-    tie_segments None when not tuned (the solver's setting is kept).
+    tie_segments None when not tuned (the solver's setting is kept), 0
+    (automatic) on a solver that takes none.
 
     Coordinate descent: the sweep shape, then the round tiles under the
     default schedule, the schedule under those tiles, the segments; then the
@@ -78,7 +78,9 @@ def autotune(solver, frames_ptr: int, nev: int, device: bool = True, repeats: in
     best = tune_tiles()
     best_sched = tune_schedule()
     best_seg = (None, best_sched[2])
-    if tune_segments:
+    if tune_segments and not getattr(solver, "takes_sweep_segments", True):
+        best_seg = (0, best_sched[2])
+    elif tune_segments:
         for ts in TIE_SEGMENTS:
             solver.set_sweep_segments(0, ts)
             ms = _time(solver, frames_ptr, nev, device, repeats)
