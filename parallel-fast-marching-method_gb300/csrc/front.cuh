@@ -202,17 +202,20 @@ __global__ void __launch_bounds__(32) front_kernel(FrontArgs<R> a)
                 for (int j = 0; j < PER; ++j)
                     wait = wait || (hok[j] && hfield[j] && front_unwritten(halo[lane + 32 * j]));
                 if (!__any_sync(0xffffffffu, wait)) break;
-                const bool give_up = wait_gives_up(++polls, a.err);
-                // (hp stands AHEAD + 1 layers above.  After another wait gave
-                // up, rows of layers above the grid, which are not copied
-                // anew, can hold unwritten values too: not polled)
+                if (wait_gives_up(++polls, a.err)) {
+                    // (none is left in the ring: rows of layers above the
+                    // grid are not copied anew, and a value unwritten there
+                    // would be polled before the field)
+#pragma unroll
+                    for (int j = 0; j < PER; ++j)
+                        if (hok[j] && hfield[j] && front_unwritten(halo[lane + 32 * j])) halo[lane + 32 * j] = INF;
+                    break;
+                }
+                // (hp stands AHEAD + 1 layers above)
 #pragma unroll
                 for (int j = 0; j < PER; ++j)
                     if (hok[j] && hfield[j] && front_unwritten(halo[lane + 32 * j]))
-                        halo[lane + 32 * j] = give_up || !halo_layer_in(t, hlate[j], nnr)
-                                                  ? INF
-                                                  : front_load(hp[j] + (AHEAD + 1) * hstep[j]);
-                if (give_up) break;
+                        halo[lane + 32 * j] = front_load(hp[j] + (AHEAD + 1) * hstep[j]);
             }
         }
         // (a ring holds more layers than a step reads, so that a lane one step

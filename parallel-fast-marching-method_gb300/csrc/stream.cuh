@@ -79,22 +79,22 @@ __device__ void stream_mark(const StreamArgs<R> &a, int e, int gr, int gx, int g
 }
 
 // Polls of a halo value or an upstream word (an L2 round trip each, about a
-// second in all; a multiple of 64) before the error flag is raised and the
-// block goes on.
+// second in all) before the error flag is raised and the block goes on.
 #ifndef FM_WAIT_POLLS
 #define FM_WAIT_POLLS (1u << 20)
 #endif
 
-// Whether a warp's wait ends unanswered after `polls` polls: its limit is
-// reached, or another wait's was, looked for every 64th poll.  The warp decides
-// as one (a vote): lanes that saw the error word change between their reads
-// would otherwise part, and wait for each other in the votes and shuffles ahead.
+// Whether a warp's wait ends unanswered after `polls` polls (the same in all
+// lanes): its limit is reached, or another wait's was, looked for every 64th
+// poll.  The lanes take one read of the error word: lanes that saw it change
+// between their reads would part, and wait for each other in the votes and
+// shuffles ahead.
 __device__ __forceinline__ bool wait_gives_up(unsigned polls, int *err)
 {
-    static_assert(FM_WAIT_POLLS % 64 == 0, "looked at every 64th poll");
-    if (polls & 63u) return false;
-    if (!__any_sync(0xffffffffu, polls >= FM_WAIT_POLLS || (*(volatile int *)err & 16))) return false;
-    if ((threadIdx.x & 31) == 0) atomicOr(err, 16);
+    if (!(polls > FM_WAIT_POLLS ||
+          ((polls & 63u) == 0u && (__shfl_sync(0xffffffffu, *(volatile int *)err, 0) & 16))))
+        return false;
+    atomicOr(err, 16);
     return true;
 }
 // Steps between two publications of a block's word.  Each costs a fence, and

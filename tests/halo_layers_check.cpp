@@ -4,10 +4,11 @@
 // halo layers used AHEAD steps later into a ring row (halo_layers.h says which
 // layers the grid has), then polls the columns whose value is unwritten.  The
 // blocks upstream write their columns' first `upto` layers and then never
-// again, so a wait gives up.  No copy and no poll may read a layer the grid
-// does not have, the sweep has to end, and the values it uses in steps after
-// the last copies must be settled ones.  With the rule left out of the polls
-// the same loop reads layers above the grid, so the check can tell.
+// again, so a wait gives up, and leaves unset what it waited for.  No copy and
+// no poll may read a layer the grid does not have, the sweep has to end, and
+// the values it uses have to be settled ones.  If a wait that gives up leaves
+// its row as it is, the same loop reads layers above the grid, so the check can
+// tell.
 //
 //   g++ -O2 -std=c++17 halo_layers_check.cpp -o check && ./check
 #include <algorithm>
@@ -26,7 +27,7 @@ struct Found {
 };
 
 // the columns of one side (n of them) of a block of sx x sz columns
-void sweep(int sx, int sz, bool skew, int n, int nnr, int upto, bool rule, Found &f)
+void sweep(int sx, int sz, bool skew, int n, int nnr, int upto, bool clear, Found &f)
 {
     const int lag = sx + sz - 2, ring = lag + kAhead + 2 <= 16 ? 16 : 32;
     std::vector<int> rows(ring * n, kUnset);
@@ -53,10 +54,10 @@ void sweep(int sx, int sz, bool skew, int n, int nnr, int upto, bool rule, Found
             for (int q = 0; q < n; ++q) {
                 int &v = rows[(t % ring) * n + q];
                 if (v != kUnwritten) continue;
-                if (rule)
-                    v = give_up || !fm3dt::halo_layer_in(t, late(q), nnr) ? kUnset : read(t - late(q));
-                else if (!give_up)
+                if (!give_up)
                     v = read(t - late(q));
+                else if (clear)
+                    v = kUnset;
             }
             if (give_up) {
                 gave_up = true;
@@ -87,7 +88,7 @@ int main()
                         sweep(s[0], s[1], skew, s[side], nnr, upto, true, with);
                         sweep(s[0], s[1], skew, s[side], nnr, upto, false, without);
                     }
-    std::printf("%lld reads, %lld outside, %lld values used, %lld unsettled; without the rule %lld outside\n", with.reads,
+    std::printf("%lld reads, %lld outside, %lld values used, %lld unsettled; left as they are, %lld outside\n", with.reads,
                 with.outside, with.used, with.unsettled, without.outside);
     return with.outside == 0 && with.unsettled == 0 && without.outside > 0 ? 0 : 1;
 }
