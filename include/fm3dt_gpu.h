@@ -308,9 +308,11 @@ int fm3dt_part_ms(fm3dt_ctx *ctx, float *ms);
  * compaction; ms[2] of the copies out; ms[3] the call's wall time. */
 int fm3dt_rays_ms(fm3dt_ctx *ctx, float *ms);
 
-/* The last solve's near-tie extra sweeps after the first skip the work items
- * (a block of columns of one event) where nothing near them changed: run[k] / skipped[k] the items extra sweep k ran and skipped,
- * for up to cap sweeps (sweep 0 runs every item and counts none).  Returns
+/* The last solve's near-tie extra sweeps skip the work items (a block of
+ * columns of one event) where nothing near them changed -- the first those where
+ * the certification of the main sweep left no node open: run[k] / skipped[k] the
+ * items extra sweep k ran and skipped, for up to cap sweeps (0 and 0 for sweep
+ * 0, whose items are not counted).  Returns
  * the number of extra sweeps recorded (0 when none tracked activity). */
 int fm3dt_tie_sweep_items(fm3dt_ctx *ctx, int cap, int64_t *run, int64_t *skipped);
 

@@ -274,8 +274,9 @@ const CUtensorMap *field_tensor_map(fm3dt_ctx *ctx, int shape)
 //   FM_TIE_QUEUE           the near-tie events' last extra sweep queues the tiles
 //                          it changes for their first round, which then takes
 //                          those tiles instead of every tile
-//   FM_TIE_SKIP            the near-tie events' extra sweeps after the first skip
-//                          the items where nothing near them changed (StreamArgs)
+//   FM_TIE_SKIP            the near-tie events' extra sweeps skip the items where
+//                          nothing near them changed (StreamArgs), the first those
+//                          that the certification of the main sweep leaves none open in
 #ifndef FM_TIE_QUEUE
 #define FM_TIE_QUEUE 1
 #endif

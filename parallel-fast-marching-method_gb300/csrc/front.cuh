@@ -39,8 +39,8 @@
 // against 228; eight 256^3 events 2.41 ms against 1.69 without it.
 //
 // What bounds it: instruction issue when there are events enough to fill the
-// SMs (82% of the issue slots, 10.0 warp instructions a node), else the step's
-// latency (~0.5 us) along the critical path.  Against one launch per
+// SMs (84% of the issue slots; 9.5 warp instructions a node with 128 layers, 9.8
+// with 96), else the step's latency (~0.5 us) along the critical path.  Against one launch per
 // hyperplane of blocks in height segments, with rings of whole layers and
 // their halos: 500 events on 192x224x224 77.8 -> 42.4 ms, 256 on 128^3 10.3 ->
 // 5.5 ms, eight on 256^3 4.26 -> 1.67 ms, one on 64^3 0.52 -> 0.19 ms; in double

@@ -5,7 +5,8 @@
 // loop with halo exchange (F:6371-6451, 6691-6892) by two device-side passes
 // over tiles of the grid:
 //
-//  1. Sweep.  Tiles are visited in wavefront order of the event's dominant
+//  1. Sweep (here by tiles; the default, by columns, is in front.cuh and
+//     stream.cuh).  Tiles are visited in wavefront order of the event's dominant
 //     propagation direction (upward from the bottom face, and along +/-theta
 //     and +/-phi as the boundary frame's gradient says): one launch per tile
 //     hyperplane, every tile's upwind neighbour tiles already done.  Inside a
@@ -177,10 +178,13 @@ struct Tile {
 };
 
 // Resident 128-thread CTAs per SM that the register allocation must allow.
-// (Rounds in single precision: 6, 80 registers, since the short form of the
-// update; with 8 and 64 registers it spills.)
-// The kernels are issue-bound with long dependent chains, so occupancy pays
-// until registers spill.
+// Rounds in single precision: 6 (80 registers, 76-104 bytes of spill loads by
+// tile shape).  With 4 (112-114 registers, no spills), 5, 6 and 8 (64 registers,
+// 200-420 bytes): two point sources on 96^3 12.5, 12.5, 12.0, 12.5 ms, twelve
+// first-order events on 75x91x83 3.08, 3.07, 3.09, 3.15, eight events with a
+// slow slab on 256^3 5.94, 5.85, 5.86, 6.01.  Double precision: 4 (128 registers,
+// 216-436 bytes); with 3 or 2 (165-199, no spills) two events on 192x224x224 136 ms
+// instead of 118, 32 on 128^3 alike.
 #ifndef FM_ROUND_MINB_F32
 #define FM_ROUND_MINB_F32 6
 #endif

@@ -258,22 +258,11 @@ FM_HD R fm_update_octants(R s, const R t1[6], const R t2[6], unsigned inb, const
     return tmin + best;
 }
 
-// The node update of a sweep from an unset field, where every neighbour
-// downstream of the sweep (up, r-1, and the lateral directions the sweep runs
-// toward) is still unset when the node is computed.  Then only the three
-// upstream neighbours -- down (r+1) and the lateral ones the sweep comes
-// from, here D, X and Z -- can enter an octant, and each of the eight octants
-// is the causal solve of the upstream terms it contains: the octant that
-// takes the upstream side on the axes of a subset S of {D, X, Z} and the
-// downstream side on the others solves S (its downstream terms are +inf,
-// sort last and never pass k < x).  So this returns fm_update's value, bit
-// for bit, with +inf at the downstream neighbours: the same keys, the same
-// stable order within each subset (key, then axis r, theta, phi), the same
-// arithmetic, and an octant counted when its three neighbours lie inside the
-// grid.  It evaluates the seven subsets with four quadratic solves instead of
-// the eight octants' sixteen: the singletons are one FMA each, the three pairs
-// one solve each, and the triple's first two terms are one of the pairs (the
-// same order and the same operations, hence the same bits), so only its
+// The least value, relative to tmin, of the causal solves of the seven subsets
+// of three sides (one an axis), with four quadratic solves instead of the eight
+// octants' sixteen: the singletons are one FMA each, the three pairs one solve
+// each, and the triple's first two terms are one of the pairs (the same order and
+// the same operations as the octants', hence the same bits), so only its
 // three-term solve is added.  The four solves are straight-line code with
 // selects at the end: a sweep's few warps wait on each other, and three pairs
 // solved side by side are a third of the chain of three branches (main sweep of
@@ -282,13 +271,8 @@ FM_HD R fm_update_octants(R s, const R t1[6], const R t2[6], unsigned inb, const
 // either order; only the innermost FMA of a pair's c depends on which term
 // comes first.
 //
-// tD/tD2, tX/tX2, tZ/tZ2: upstream first and second neighbour values;
-// in*: whether each upstream (u) and downstream (d) neighbour lies inside the
-// grid (inD: r+1, inU: r-1).
-// The seven subsets' least value, relative to tmin (the least of the three
-// times): t1, t2 the three sides' first and second neighbour values (D, X, Z
-// above), n / f: whether each of these sides, and the opposite one, lies inside
-// the grid.
+// t1, t2: the sides' first and second neighbour values; tmin: the least of t1;
+// n / f: whether each side, and the opposite one, lies inside the grid.
 template <typename R>
 FM_HD R fm_subsets(R s, const R t1[3], const R t2[3], R tmin, bool n0, bool f0, bool n1, bool f1, bool n2, bool f2,
                    const Spacing<R> &sp, int order2)
@@ -359,6 +343,23 @@ FM_HD R fm_subsets(R s, const R t1[3], const R t2[3], R tmin, bool n0, bool f0, 
     return best;
 }
 
+// The node update of a sweep from an unset field, where every neighbour
+// downstream of the sweep (up, r-1, and the lateral directions the sweep runs
+// toward) is still unset when the node is computed.  Then only the three
+// upstream neighbours -- down (r+1) and the lateral ones the sweep comes
+// from, here D, X and Z -- can enter an octant, and each of the eight octants
+// is the causal solve of the upstream terms it contains: the octant that
+// takes the upstream side on the axes of a subset S of {D, X, Z} and the
+// downstream side on the others solves S (its downstream terms are +inf,
+// sort last and never pass k < x).  So this returns fm_update's value, bit
+// for bit, with +inf at the downstream neighbours: the same keys, the same
+// stable order within each subset (key, then axis r, theta, phi), the same
+// arithmetic, and an octant counted when its three neighbours lie inside the
+// grid.
+//
+// tD/tD2, tX/tX2, tZ/tZ2: upstream first and second neighbour values;
+// in*: whether each upstream (u) and downstream (d) neighbour lies inside the
+// grid (inD: r+1, inU: r-1).
 template <typename R>
 FM_HD R fm_update_upstream(R s, R tD, R tD2, R tX, R tX2, R tZ, R tZ2, bool inD, bool inU, bool inXu, bool inXd,
                            bool inZu, bool inZd, const Spacing<R> &sp, int order2)

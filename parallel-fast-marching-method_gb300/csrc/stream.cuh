@@ -34,8 +34,12 @@
 // published word tells before the step.  Quiet chunks are passed by without
 // loading them.
 //
-// What bounds it is the chain: nnr steps and a block's lag for every hyperplane
-// of blocks, SX steps along theta and SZ along phi (and the publication's).
+// What bounds it with few events is the chain: nnr steps and a block's lag for
+// every hyperplane of blocks, SX steps along theta and SZ along phi (and the
+// publication's).  With many (141 near ties on 96x112x112) it is throughput, by
+// the blocks and steps that run: 55-63% of the issue slots in the sweeps that
+// run most blocks, from the 15.5 warps an SM that 128 registers allow, which
+// wait for their own instructions; DRAM 2-6%.
 // With whole layers instead of steps in the words, a block lagged SX + SZ - 1
 // steps along either: two double-precision events on 192x224x224 131 -> 120.5 ms,
 // 32 on 128^3 22.9 -> 21.4, 500 single-precision ones on 192x224x224 94.5 ->
