@@ -649,7 +649,9 @@ __global__ void __launch_bounds__(256) certify_kernel(const CertifyArgs<R> a)
     int next = g0;                                  // the next layer copied; src stands at it
     auto plane = [&](int row) {
         R *d = &s_plane[row][tid];
-        const bool set = next < f.nnr;
+        // (no further than the last node's second neighbour: nothing copies
+        // into a block that has ended)
+        const bool set = next < min(f.nnr, g1 + 2);
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
             if (in[j]) {
